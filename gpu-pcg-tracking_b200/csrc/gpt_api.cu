@@ -706,6 +706,7 @@ static gpt_status setup_batch(gpt_handle *h, uint32_t B, const uint32_t *Ns, con
     bv.knot_off = h->knot_off;
     bv.knot_inst = h->knot_inst;
     bv.st = h->st;
+    bv.part_warps = part_warps((int)B, maxN, h->num_sms);
     maxN_out = maxN;
     minN_out = minN;
     return GPT_OK;

@@ -57,6 +57,9 @@ struct BatchView {
     // A view of a contiguous sub-range of a batch: instances b0 .. b0+B-1, owning knots
     // j0 .. j0+total_knots-1.  Instance and knot indices stay those of the whole batch.
     int j0 = 0, b0 = 0;
+    // the partitioned PCG's warps per instance, fixed by the whole batch so that its parts give the same bits
+    // (0: by this view)
+    int part_warps = 0;
 
     __device__ __forceinline__ int inst(int j) const { return knot_inst ? knot_inst[j] : 0; }
     __device__ __forceinline__ int off(int b) const { return knot_off ? knot_off[b] : 0; }

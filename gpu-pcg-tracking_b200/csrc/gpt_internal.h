@@ -12,7 +12,7 @@ constexpr int MAX_PCG_KNOTS = 512;  // horizon limit of the library (16-CTA clus
 constexpr int PCG_KPC_MAX = 128;    // knots per CTA held in shared memory by the PCG
 constexpr int PCG_KPC_STAIR = 64;   // with the stair preconditioner (its Pinv blocks staged too)
 constexpr int PCG_WARP_PAIR = 32;   // pcg_cluster_size value selecting pcg_pair_kernel (one 128-thread CTA per instance)
-constexpr int PCG_WARP_QUAD = 64;   // pcg_cluster_size value selecting pcg_quad_kernel (four warps factor four parts)
+constexpr int PCG_WARP_QUAD = 64;   // pcg_cluster_size value selecting pcg_part_kernel (the warps factor parts of the horizon)
 
 // SQP control constants (settings.cuh:31-50 and the -D flags of perform_experiment.sh:42-58)
 struct SolverParams {
@@ -64,6 +64,13 @@ cudaError_t launch_pcg(const BatchView &bv, int max_n_knots, int min_n_knots, in
                        const float *Pinv, const float *gamma, const double *gamma64, float *lambda, double *lambda64,
                        double *cr_ws, int max_iter, float tol, int exit_mode, uint32_t *out_iters, uint32_t *pcg_log,
                        int log_stride, int cluster_size, int num_sms, cudaStream_t s);
+// the partitioned kernel of cluster_size PCG_WARP_QUAD (gpt_part.cu; fmt 1 or 2, exact preconditioner)
+cudaError_t launch_pcg_part(const BatchView &bv, int max_n, int fmt, const void *S, const float *gamma,
+                            const double *gamma64, float *lambda, double *lambda64, double *ws, int max_iter,
+                            float tol, int exit_mode, uint32_t *out_iters, uint32_t *pcg_log, int log_stride,
+                            int num_sms, cudaStream_t s);
+// its warps per instance for a batch of B instances (BatchView::part_warps carries it to part-batch views)
+int part_warps(int B, int max_n, int num_sms);
 // lambda64 (optional) replaces lambda when given; Ginv64c (optional): the compact inverses of
 // launch_schur64 (GC64 doubles per knot), with Ginv64 holding only the blocks its flags name
 cudaError_t launch_dz(const BatchView &bv, const float *Ginv, const double *Ginv64, const double *Ginv64c,

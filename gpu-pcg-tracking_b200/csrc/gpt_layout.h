@@ -1,5 +1,5 @@
-// gpt_layout.h -- the part layout of the partitioned PCG (pcg_quad_kernel): which knots each of
-// the four factoring warps owns and where the separator knots lie.  Plain C++ (host and device), so
+// gpt_layout.h -- the part layout of the partitioned PCG (pcg_part_kernel): which knots each of
+// the factoring warps owns and where the separator knots lie.  Plain C++ (host and device), so
 // the CPU tests compile it and check the layout for every horizon.
 #pragma once
 
@@ -13,45 +13,51 @@ namespace gpt {
 
 constexpr int QUAD_NWARP = 4;
 
-struct QuadLayout {
+// NW: the most parts; edge: an edge part's length in tenths of a middle part's
+template <int NW>
+struct PartLayout {
     int P;
-    int a[QUAD_NWARP], b[QUAD_NWARP];  // part p: knots a[p] .. b[p] (b[p] < a[p]: empty)
-    int s[QUAD_NWARP - 1];             // separator knots
+    int a[NW], b[NW];  // part p: knots a[p] .. b[p] (b[p] < a[p]: empty)
+    int s[NW - 1];     // separator knots
 };
-GPT_HD inline QuadLayout quad_layout(int n)
+template <int NW>
+GPT_HD inline PartLayout<NW> part_layout(int n, int edge)
 {
-    QuadLayout L;
-    int P = QUAD_NWARP;
+    PartLayout<NW> L;
+    int P = NW;
     if (n < 2 * P) {
         P = (n + 1) / 2;
-        P = P < 1 ? 1 : (P > QUAD_NWARP ? QUAD_NWARP : P);
+        P = P < 1 ? 1 : (P > NW ? NW : P);
     }
     L.P = P;
     const int nint = n - (P - 1);
-    int len[QUAD_NWARP] = {0, 0, 0, 0};
+    int len[NW] = {};
     if (P == 1) {
         len[0] = n;
     } else if (P == 2) {
         len[0] = nint / 2;
         len[1] = nint - len[0];
     } else {
-        const int y = (10 * nint) / (26 + 10 * (P - 2));  // edge parts weighted 1.3
+        const int y = (10 * nint) / (2 * edge + 10 * (P - 2));
         const int rest = nint - (P - 2) * y;
         len[0] = rest / 2;
         for (int p = 1; p < P - 1; ++p) len[p] = y;
         len[P - 1] = rest - len[0];
     }
     int pos = 0;
-    for (int p = 0; p < QUAD_NWARP; ++p) {
+    for (int p = 0; p < NW; ++p) {
         L.a[p] = pos;
         L.b[p] = pos + (p < P ? len[p] : 0) - 1;
         pos += p < P ? len[p] : 0;
-        if (p < QUAD_NWARP - 1) {
+        if (p < NW - 1) {
             L.s[p] = pos;
             if (p < P - 1) ++pos;
         }
     }
     return L;
 }
+
+using QuadLayout = PartLayout<QUAD_NWARP>;
+GPT_HD inline QuadLayout quad_layout(int n) { return part_layout<QUAD_NWARP>(n, 13); }
 
 }  // namespace gpt

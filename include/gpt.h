@@ -84,7 +84,7 @@ typedef struct gpt_solver_config {
     float rho_max;             /* RHO_MAX */
     float rho_min;             /* RHO_MIN */
     uint32_t pcg_cluster_size; /* CTAs per instance in the PCG (1,2,4,8,16); GPT_PCG_WARP_PAIR / GPT_PCG_WARP_QUAD:
-                                  one 128-thread CTA per instance, factorisation by two / four warps (pcg_precond 1
+                                  one CTA per instance, factorisation from both ends / in parts (pcg_precond 1
                                   only); 0 = chosen by the library (gpt_autotune's choice for the batch shape, else
                                   1 ... 16) */
     uint32_t pcg_precond;      /* 0: block-Jacobi Pinv (the reference's, oldschur.cuh:926-933);
@@ -120,10 +120,12 @@ typedef struct gpt_sqp_stats {
  * concurrently; same iteration and preconditioner (exact inverse of S) as pcg_cluster_size 1. */
 #define GPT_PCG_WARP_PAIR 32u
 
-/* pcg_cluster_size value: the PCG of one instance in one 128-thread CTA whose four warps each factor about a
- * quarter of the horizon (partitioned block LDL^T: three separator knots, a 3-block reduced system), so every
- * SM sub-partition factors and each warp's chain is half the warp-pair kernel's; same iteration and
- * preconditioner (exact inverse of S) as pcg_cluster_size 1. */
+/* pcg_cluster_size value: the PCG of one instance in one CTA whose warps each factor a part of the horizon
+ * (partitioned block LDL^T: separator knots between the parts, whose reduced system one warp factors), with
+ * 8, 4 or 2 warps by the batch size and the longest horizon of the call (few instances: more warps, a
+ * shorter chain; many: less work); same iteration and preconditioner (exact inverse of S) as
+ * pcg_cluster_size 1.  The same batch gives the same bits; an instance's last bits may differ between
+ * batches that run with another number of warps. */
 #define GPT_PCG_WARP_QUAD 64u
 
 /* Default configs: the reference's logged experiment settings (dt 1/64, Euler,
