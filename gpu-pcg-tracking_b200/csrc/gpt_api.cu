@@ -564,6 +564,12 @@ gpt_status gpt_pcg(gpt_handle *h, uint32_t N, const float *d_S, const float *d_P
         GPT_CUDA(launch_pcg(single_view(N), (int)N, (int)N, 2, 1, reinterpret_cast<const float *>(h->S64), d_Pinv,
                             d_gamma, h->gamma64, d_lambda, d_lambda64, h->crw, (int)max_iter, tol, (int)exit_mode,
                             h->pcg_out, nullptr, 0, (int)h->sc.pcg_cluster_size, h->num_sms, s));
+    } else if (h->sc.pcg_cluster_size == 0 && h->sc.pcg_precond == 1) {
+        // the library's choice: the partitioned kernel on the same conversion, from the caller's lambda (N = 100:
+        // 130 -> 75 us against cyclic reduction on the caller's rows)
+        GPT_CUDA(launch_pack_rows64((int)N, d_S, d_gamma, h->S64, h->gamma64, h->num_sms, s));
+        GPT_CUDA(launch_pcg_part(single_view(N), (int)N, 2, h->S64, d_gamma, h->gamma64, d_lambda, d_lambda64, h->crw,
+                                 (int)max_iter, tol, (int)exit_mode, h->pcg_out, nullptr, 0, h->num_sms, s, true));
     } else {
         GPT_CUDA(launch_pcg(single_view(N), (int)N, (int)N, 0, (int)h->sc.pcg_precond, d_S, d_Pinv, d_gamma, nullptr,
                             d_lambda, d_lambda64, h->crw, (int)max_iter, tol, (int)exit_mode, h->pcg_out, nullptr, 0,

@@ -64,11 +64,12 @@ cudaError_t launch_pcg(const BatchView &bv, int max_n_knots, int min_n_knots, in
                        const float *Pinv, const float *gamma, const double *gamma64, float *lambda, double *lambda64,
                        double *cr_ws, int max_iter, float tol, int exit_mode, uint32_t *out_iters, uint32_t *pcg_log,
                        int log_stride, int cluster_size, int num_sms, cudaStream_t s);
-// the partitioned kernel of cluster_size PCG_WARP_QUAD (gpt_part.cu; fmt 1 or 2, exact preconditioner)
+// the partitioned kernel of cluster_size PCG_WARP_QUAD (gpt_part.cu; fmt 1 or 2, exact preconditioner); warm:
+// start from lambda instead of 0
 cudaError_t launch_pcg_part(const BatchView &bv, int max_n, int fmt, const void *S, const float *gamma,
                             const double *gamma64, float *lambda, double *lambda64, double *ws, int max_iter,
                             float tol, int exit_mode, uint32_t *out_iters, uint32_t *pcg_log, int log_stride,
-                            int num_sms, cudaStream_t s);
+                            int num_sms, cudaStream_t s, bool warm = false);
 // its warps per instance for a batch of B instances (BatchView::part_warps carries it to part-batch views)
 int part_warps(int B, int max_n, int num_sms);
 // lambda64 (optional) replaces lambda when given; Ginv64c (optional): the compact inverses of

@@ -3,7 +3,7 @@
 //
 // Solves S lambda = gamma by conjugate gradients with the exact inverse of S as the preconditioner
 // (z = S^{-1} r up to rounding), so the iteration stops after one step; it starts from lambda = 0
-// (r_0 = gamma: a warm start cannot save the one step).  With M = -S (SPD), A_k = M_kk and
+// (r_0 = gamma: a warm start cannot save the one step) unless asked to start from the given lambda.  With M = -S (SPD), A_k = M_kk and
 // E_k = M_{k,k-1} = -L_k (L_k the left block of row k of S), the horizon is cut by P - 1 separator
 // knots s_1 < ... < s_{P-1} into P parts.  Part 0 is eliminated top-down toward s_1 and part P-1
 // bottom-up toward s_{P-1}; a middle part top-down from its left to its right separator, which couples
@@ -466,7 +466,7 @@ struct PartArgs {
     const double *gamma64;
     float *lambda;
     double *lambda64, *ws;
-    int max_iter, exit_mode, log_stride;
+    int max_iter, exit_mode, log_stride, warm;
     float tol;
     uint32_t *out_iters, *pcg_log;
 };
@@ -753,7 +753,27 @@ __global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const _
     }
     int it = 0, set = 0;
     bool conv = false, bad = false, in_xv = false;
+    bool has_res = false;  // r and lambda are in the workspace (before: r = gamma, lambda = 0)
     double eta = 0.0, gg = 0.0, alpha = 0.0;
+    if (A.warm) {
+        const PartCtx<FMT, CF> cx(A);
+        double g2[2] = {0.0, 0.0};  // gamma . gamma; entries of lambda that are not 0
+        for (int e = tid; e < NS * cx.n; e += NT) {
+            const double lam = (double)A.lambda[NS * cx.kg0 + e];
+            cx.vec(QW_LAM, e) = lam;
+            g2[0] = fma(xv[e], xv[e], g2[0]);
+            g2[1] += lam != 0.0 ? 1.0 : 0.0;
+        }
+        part_sum<CF, 2>(g2, set);
+        if (g2[1] > 0.0) {
+            gg = g2[0];
+            part_true_residual<FMT, CF>(A, set ^ 1);
+            for (int e = tid; e < NS * cx.n; e += NT) xv[e] = cx.vec(QW_RES, e);
+            has_res = true;
+        } else {
+            set ^= 1;
+        }
+    }
     auto converged = [&](double e, double r2) {
         return A.exit_mode == 0 ? (r2 <= (double)A.tol * (double)A.tol * gg) : (fabs(e) < (double)A.tol);
     };
@@ -763,7 +783,7 @@ __global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const _
         const int nv = NS * cx.n;
         double dd[3] = {0.0, 0.0, 0.0};  // r . z, r . r with z = -x; x . S x
         for (int e = tid; e < nv; e += NT) {
-            const double r = it > 0 ? cx.vec(QW_RES, e) : cx.gam(e), x = xv[e];
+            const double r = has_res ? cx.vec(QW_RES, e) : cx.gam(e), x = xv[e];
             dd[0] = fma(-x, r, dd[0]);
             dd[1] = fma(r, r, dd[1]);
             dd[2] = fma(x, cx.vec(QW_SX, e), dd[2]);
@@ -771,8 +791,8 @@ __global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const _
         part_sum<CF, 3>(dd, set);
         set ^= 1;
         if (it == 0) {
-            gg = dd[1];
-            conv = converged(dd[0], gg);
+            if (!has_res) gg = dd[1];
+            conv = converged(dd[0], dd[1]);
         } else {
             if (!isfinite(dd[0])) {
                 bad = true;
@@ -806,22 +826,23 @@ __global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const _
         }
         double r2[1] = {0.0};
         for (int e = tid; e < nv; e += NT) {
-            const double rn = fma(alpha, cx.vec(QW_SX, e), it > 0 ? cx.vec(QW_RES, e) : cx.gam(e));
+            const double rn = fma(alpha, cx.vec(QW_SX, e), has_res ? cx.vec(QW_RES, e) : cx.gam(e));
             r2[0] = fma(rn, rn, r2[0]);
         }
         part_sum<CF, 1>(r2, set);
         set ^= 1;
         ++it;
-        if (it == 1 && A.exit_mode == 0 && converged(0.0, r2[0])) {
+        if (!has_res && A.exit_mode == 0 && converged(0.0, r2[0])) {
             conv = in_xv = true;  // lambda = alpha p
             break;
         }
         for (int e = tid; e < nv; e += NT) {
-            cx.vec(QW_RES, e) = fma(alpha, cx.vec(QW_SX, e), it > 1 ? cx.vec(QW_RES, e) : cx.gam(e));
-            cx.vec(QW_LAM, e) = fma(-alpha, xv[e], it > 1 ? cx.vec(QW_LAM, e) : 0.0);
+            cx.vec(QW_RES, e) = fma(alpha, cx.vec(QW_SX, e), has_res ? cx.vec(QW_RES, e) : cx.gam(e));
+            cx.vec(QW_LAM, e) = fma(-alpha, xv[e], has_res ? cx.vec(QW_LAM, e) : 0.0);
             cx.vec(QW_P, e) = -xv[e];
             cx.vec(QW_V, e) = -cx.vec(QW_SX, e);
         }
+        has_res = true;
         bool replaced = false;
         if (it % RR_PERIOD == 0) {
             r2[0] = part_true_residual<FMT, CF>(A, set);
@@ -846,7 +867,7 @@ __global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const _
     }
     const PartCtx<FMT, CF> cx(A);
     for (int e = tid; e < NS * cx.n; e += NT) {
-        const double lam = in_xv ? -alpha * xv[e] : (it > 0 ? cx.vec(QW_LAM, e) : 0.0);
+        const double lam = in_xv ? -alpha * xv[e] : (has_res ? cx.vec(QW_LAM, e) : 0.0);
         A.lambda[NS * cx.kg0 + e] = (float)lam;
         if (A.lambda64) A.lambda64[NS * cx.kg0 + e] = lam;
     }
@@ -907,10 +928,10 @@ static cudaError_t launch_part_f(const PartArgs &A, int max_n, int fmt, cudaStre
 cudaError_t launch_pcg_part(const BatchView &bv, int max_n, int fmt, const void *S, const float *gamma,
                             const double *gamma64, float *lambda, double *lambda64, double *ws, int max_iter,
                             float tol, int exit_mode, uint32_t *out_iters, uint32_t *pcg_log, int log_stride,
-                            int num_sms, cudaStream_t s)
+                            int num_sms, cudaStream_t s, bool warm)
 {
     const PartArgs A{bv,       S,         gamma,      gamma64, lambda,    lambda64, ws,
-                     max_iter, exit_mode, log_stride, tol,     out_iters, pcg_log};
+                     max_iter, exit_mode, log_stride, warm ? 1 : 0, tol, out_iters, pcg_log};
     switch (bv.part_warps ? bv.part_warps : part_warps(bv.B, max_n, num_sms)) {
     case 8: return launch_part_f<Part8>(A, max_n, fmt, s);
     case 4: return launch_part_f<Part4>(A, max_n, fmt, s);

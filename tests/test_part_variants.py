@@ -91,3 +91,33 @@ def test_part_variants_solve_the_system(problem_mod, sms, more, pattern, tol, mo
         for b in {i, len(pattern) * ((B - 1 - i) // len(pattern)) + i}:  # the first and last instance of this horizon
             assert check.rel_err(got[14 * off[b]:14 * off[b + 1]], want) <= 1e-6, (n, b)
     sv.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [2, 3, 33, 64, 129])
+def test_pcg_entry_point_starts_from_the_given_lambda(oracle, problem_mod, N):
+    """gpt_pcg with the library's choice of kernel: from any start it reaches the FP64 Cholesky solution, and from a
+    solution it takes no iteration and returns it unchanged (the solution rounded to float32 keeps a residual of
+    about 6e-8 x |S| |lambda| / |gamma|, far above any tolerance a user sets, so that start is checked with a
+    tolerance above it)."""
+    import torch
+    gpt = importlib.import_module("gpu-pcg-tracking_b200")
+    p = problem_mod.make_problem(N, 70 + N, dt=0.01)
+    par = oracle.make_params(dt=0.01, integrator=1, qd_cost=1e-2, r_cost=1e-4)
+    S, Pv, gam, _ = oracle.form_schur(N, 1e-2, *(np.asarray(x, np.float32) for x in oracle.form_kkt(
+        par, N, p["xu"], p["goal"], p["xs"])))
+    S, Pv, gam = (np.asarray(x, np.float32) for x in (S, Pv, gam))
+    ref = oracle.banded_cholesky(N, S.astype(np.float64), gam.astype(np.float64))
+    dev = lambda a: torch.as_tensor(np.ascontiguousarray(a, np.float32), device="cuda")  # noqa: E731
+    sv = gpt.Solver(max_knot_points=N, **SPEC_CFG)
+    rng = np.random.default_rng(N)
+    for start in (np.zeros(14 * N), rng.normal(0, np.abs(ref).max(), 14 * N), ref):
+        lam, lam64 = dev(start), torch.zeros(14 * N, device="cuda", dtype=torch.float64)
+        it, maxed = sv.pcg(N, dev(S), dev(Pv), dev(gam), lam, 50, 1e-9, 0, lam64=lam64)
+        assert not maxed and it <= 3
+        assert np.abs(lam64.cpu().numpy() - ref).max() <= 1e-6 * np.abs(ref).max()
+    lam, lam64 = dev(ref), torch.zeros(14 * N, device="cuda", dtype=torch.float64)
+    it, maxed = sv.pcg(N, dev(S), dev(Pv), dev(gam), lam, 50, 1e3, 0, lam64=lam64)
+    assert it == 0 and not maxed
+    assert np.array_equal(lam.cpu().numpy(), ref.astype(np.float32))
+    sv.close()
