@@ -732,7 +732,8 @@ static gpt_status enqueue_prologue(gpt_handle *h, const SqpPlan &pl, const float
 {
     PhaseTimer t(h, s, GPT_PHASE_INIT);
     GPT_CUDA(launch_init(pl.bv, d_xu, h->xs, pl.ns, s));
-    GPT_CUDA(launch_kkt_gconst(pl.bv, pl.P, h->G, pl.ns, s));  // G's weight-only entries, once per solve
+    if (!(pl.SP.pcg_precond == 1 && pl.SP.schur_fp64))  // G's weight-only entries, once per solve
+        GPT_CUDA(launch_kkt_gconst(pl.bv, pl.P, h->G, pl.ns, s));
     GPT_CUDA(launch_merit(pl.bv, pl.P, 1, d_xu, nullptr, d_goal, h->xs, h->knot_merit, pl.ns, s,
                           ctas_or_default(pl.SP.cta_merit)));
     GPT_CUDA(launch_accept(pl.bv, 0, pl.SP, h->knot_merit, nullptr, nullptr, nullptr, nullptr, pl.ns, s));
@@ -754,13 +755,13 @@ static gpt_status enqueue_iteration(gpt_handle *h, const SqpPlan &pl, const floa
     {
         PhaseTimer t(h, s, GPT_PHASE_KKT);
         GPT_CUDA(launch_kkt(bv, pl.P, d_xu, d_goal, h->xs, h->G, h->C, h->g, h->c, ns, s, ctas_or_default(SP.cta_kkt),
-                            false));
+                            f64 ? KKT_G_NONE : KKT_G_POS));
     }
     {
         PhaseTimer t(h, s, GPT_PHASE_SCHUR);
         if (f64) {
-            GPT_CUDA(launch_schur64(bv, h->G, h->C, h->g, h->c, h->S64, h->gamma64, nullptr, h->Ginv64, h->Ginv64c,
-                                    ns, s, ctas_or_default(SP.cta_schur)));
+            GPT_CUDA(launch_schur64(bv, pl.P, h->C, h->g, h->c, h->S64, h->gamma64, h->Ginv64c, ns, s,
+                                    ctas_or_default(SP.cta_schur)));
         } else if (stair) {
             // the reference's rows and block-Jacobi Pinv (gato_form_schur_jacobi), then the stair blocks
             if (!h->Sref) return set_err(GPT_ERR_BAD_ARG, "pcg_precond 2 was not configured on this handle");
@@ -1269,10 +1270,9 @@ gpt_status gpt_sqp_adjoint(gpt_handle *h, uint32_t B, const uint32_t *h_N, const
     const int fmt = f64 ? 2 : 1;
     GPT_CUDA(cudaMemcpyAsync(h->xs, d_xs, sizeof(float) * NS * B, cudaMemcpyDeviceToDevice, s));
     // ---- the step at xu: K [dz; lambda] = [g; c]
-    GPT_CUDA(launch_kkt(bv, P, d_xu, d_goal, h->xs, h->G, h->C, h->g, h->c, ns, s));
+    GPT_CUDA(launch_kkt(bv, P, d_xu, d_goal, h->xs, h->G, h->C, h->g, h->c, ns, s, 16, f64 ? KKT_G_NONE : KKT_G_FULL));
     if (f64)
-        GPT_CUDA(launch_schur64(bv, h->G, h->C, h->g, h->c, h->S64, h->gamma64, nullptr, h->Ginv64, h->Ginv64c, ns,
-                                s));
+        GPT_CUDA(launch_schur64(bv, P, h->C, h->g, h->c, h->S64, h->gamma64, h->Ginv64c, ns, s));
     else
         GPT_CUDA(launch_schur(1, bv, 0.f, h->G, h->C, h->g, h->c, h->S, nullptr, h->gamma, h->Ginv, h->Ginv64,
                               nullptr, SP.pcg_precond == 0 ? 1 : 0, ns, s));
@@ -1284,13 +1284,12 @@ gpt_status gpt_sqp_adjoint(gpt_handle *h, uint32_t B, const uint32_t *h_N, const
     GPT_CUDA(launch_dz(bv, h->Ginv, h->Ginv64, f64 ? h->Ginv64c : nullptr, h->C, h->g, nullptr, h->lam64, h->dz, ns,
                        s));
     if (d_xu_next) GPT_CUDA(launch_axpy(nz, -1.f, h->dz, d_xu, d_xu_next, ns, s));
-    // ---- adjoint solve K mu = [h; 0], h = dl/d(dz) = -dl/dxu+; same S (recomputed), new gamma
+    // ---- adjoint solve K mu = [h; 0], h = dl/d(dz) = -dl/dxu+; same S, new gamma
     GPT_CUDA(cudaMemsetAsync(h->adj_h, 0, sizeof(float) * NX * T, s));
     GPT_CUDA(launch_axpy(nz, -1.f, d_grad_xu_next, nullptr, h->adj_h, ns, s));
-    GPT_CUDA(cudaMemsetAsync(h->adj_zero, 0, sizeof(float) * NS * T, s));
+    if (!f64) GPT_CUDA(cudaMemsetAsync(h->adj_zero, 0, sizeof(float) * NS * T, s));
     if (f64)
-        GPT_CUDA(launch_schur64(bv, h->G, h->C, h->adj_h, h->adj_zero, h->S64, h->adj_gamma64, nullptr, h->Ginv64,
-                                h->Ginv64c, ns, s));
+        GPT_CUDA(launch_schur64_gamma(bv, h->S64, h->Ginv64c, h->C, h->adj_h, nullptr, h->adj_gamma64, ns, s));
     else
         GPT_CUDA(launch_schur(1, bv, 0.f, h->G, h->C, h->adj_h, h->adj_zero, h->S, nullptr, h->adj_gamma, h->Ginv,
                               h->Ginv64, nullptr, SP.pcg_precond == 0 ? 1 : 0, ns, s));
@@ -1418,10 +1417,10 @@ static gpt_status enqueue_track_adjoint(gpt_handle *h, const SqpPlan &pl, float 
     const int fmt = f64 ? 2 : 1;
     GPT_CUDA(launch_track_adj_begin(bv, h->trk_rows, h->trk_clk, h->trk_stbak, s));
     // the step at the solution: K [dz; lambda] = [g; c]
-    GPT_CUDA(launch_kkt(bv, pl.P, h->gxu, h->ggoal, h->xs, h->G, h->C, h->g, h->c, ns, s));
+    GPT_CUDA(launch_kkt(bv, pl.P, h->gxu, h->ggoal, h->xs, h->G, h->C, h->g, h->c, ns, s, 16,
+                        f64 ? KKT_G_NONE : KKT_G_FULL));
     if (f64)
-        GPT_CUDA(launch_schur64(bv, h->G, h->C, h->g, h->c, h->S64, h->gamma64, nullptr, h->Ginv64, h->Ginv64c, ns,
-                                s));
+        GPT_CUDA(launch_schur64(bv, pl.P, h->C, h->g, h->c, h->S64, h->gamma64, h->Ginv64c, ns, s));
     else
         GPT_CUDA(launch_schur(1, bv, 0.f, h->G, h->C, h->g, h->c, h->S, nullptr, h->gamma, h->Ginv, h->Ginv64,
                               nullptr, SP.pcg_precond == 0 ? 1 : 0, ns, s));
@@ -1435,10 +1434,9 @@ static gpt_status enqueue_track_adjoint(gpt_handle *h, const SqpPlan &pl, float 
     // the adjoint solve K mu = [h; 0], h = dl/d(dz)
     GPT_CUDA(cudaMemsetAsync(h->adj_h, 0, sizeof(float) * NX * T, s));
     GPT_CUDA(launch_track_loss_grad(bv, h->gxu, h->dz, h->ggoal, h->adj_h, h->trk_kloss, ns, s));
-    GPT_CUDA(cudaMemsetAsync(h->adj_zero, 0, sizeof(float) * NS * T, s));
+    if (!f64) GPT_CUDA(cudaMemsetAsync(h->adj_zero, 0, sizeof(float) * NS * T, s));
     if (f64)
-        GPT_CUDA(launch_schur64(bv, h->G, h->C, h->adj_h, h->adj_zero, h->S64, h->adj_gamma64, nullptr, h->Ginv64,
-                                h->Ginv64c, ns, s));
+        GPT_CUDA(launch_schur64_gamma(bv, h->S64, h->Ginv64c, h->C, h->adj_h, nullptr, h->adj_gamma64, ns, s));
     else
         GPT_CUDA(launch_schur(1, bv, 0.f, h->G, h->C, h->adj_h, h->adj_zero, h->S, nullptr, h->adj_gamma, h->Ginv,
                               h->Ginv64, nullptr, SP.pcg_precond == 0 ? 1 : 0, ns, s));

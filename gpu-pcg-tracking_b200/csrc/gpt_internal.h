@@ -39,11 +39,12 @@ inline int ctas_or_default(uint8_t v) { return v ? (int)v : 16; }
 // when handles live on several devices.
 cudaError_t ensure_func_attrs(const void *func, size_t smem_bytes, bool cluster16 = false);
 
-// full_g false: only the position block of each Q_k is written (the SQP loop, after launch_kkt_gconst
-// wrote the rest of G for the same view and weights)
+// What kkt_kernel writes of G: nothing (the FP64 Schur complement forms the cost blocks from g), the position block
+// of each Q_k (after launch_kkt_gconst wrote the rest for the same view and weights), or everything
+constexpr int KKT_G_NONE = 0, KKT_G_POS = 1, KKT_G_FULL = 2;
 cudaError_t launch_kkt(const BatchView &bv, const ProblemParams &P, const float *xu, const float *goal,
                        const float *xs, float *G, float *C, float *g, float *c, int num_sms, cudaStream_t s,
-                       int ctas_per_sm = 16, bool full_g = true);
+                       int ctas_per_sm = 16, int g_mode = KKT_G_FULL);
 cudaError_t launch_kkt_gconst(const BatchView &bv, const ProblemParams &P, float *G, int num_sms, cudaStream_t s);
 // Ginv64 (optional) receives the inverses in FP64; need_pinv = 0 skips the theta inversion in mode 1
 cudaError_t launch_schur(int mode, const BatchView &bv, float rho_scalar, const float *G, const float *C,
@@ -84,13 +85,15 @@ cudaError_t launch_accept(const BatchView &bv, int mode, const SolverParams &SP,
                           const float *dz, float *xu, float *merits_out, uint32_t *active_count, int num_sms,
                           cudaStream_t s);
 cudaError_t launch_init(const BatchView &bv, const float *xu, float *xs, int num_sms, cudaStream_t s);
-// FP64 Schur complement for the exact-preconditioner PCG: packed rows (PK64 doubles per knot), gamma
-// (FP64), the inverses in compact form (Ginv64c, GC64 doubles per knot; a block that is not
-// (block) diagonal in the full layout of Ginv64 instead; Ginv FP32 in the full layout too when
-// non-null); rho from bv.st
-cudaError_t launch_schur64(const BatchView &bv, const float *G, const float *C, const float *g, const float *c,
-                           double *S64, double *gamma64, float *Ginv, double *Ginv64, double *Ginv64c, int num_sms,
-                           cudaStream_t s, int ctas_per_sm = 16);
+// FP64 Schur complement for the exact-preconditioner PCG (gpt_schur64.cu) from kkt_kernel's C, g, c and the cost
+// weights of P: packed rows (PK64 doubles per knot), gamma (FP64), the inverses in compact form (Ginv64c, GC64
+// doubles per knot); rho from bv.st
+cudaError_t launch_schur64(const BatchView &bv, const ProblemParams &P, const float *C, const float *g, const float *c,
+                           double *S64, double *gamma64, double *Ginv64c, int num_sms, cudaStream_t s,
+                           int ctas_per_sm = 16);
+// the right-hand side of the rows and inverses it left, for another gradient g and defect c (null: 0)
+cudaError_t launch_schur64_gamma(const BatchView &bv, const double *S64, const double *Ginv64c, const float *C,
+                                 const float *g, const float *c, double *gamma64, int num_sms, cudaStream_t s);
 // adjoint of the SQP step (gpt_adjoint.cu): per-knot goal gradients, per-instance weight gradients;
 // part holds adjoint_part_floats() floats per knot
 // (wacc non-null: the 15 weight gradients of each active instance are added to wacc[15 b ..] instead of

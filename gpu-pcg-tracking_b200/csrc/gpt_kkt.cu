@@ -14,9 +14,10 @@
 // and writes the reference blocks G_k = {Q_k, R_k}, C_k = {-A_k, -B_k},
 // g_k = {q_k, r_k}, c_{k+1}.  The half-warp of knot N-2 also writes the terminal
 // Q_{N-1}, q_{N-1} and c_0 = x_0 - x_s (schur.cuh:429-479).  Inside the SQP loop
-// (FULL_G false) only the knot-dependent 7x7 position block of Q_k is written: the
-// rest of G (the velocity diagonal, R, the zeros) depends on the cost weights only and
-// is written once per solve by gconst_kernel.
+// nothing of G is written (KKT_G_NONE: the FP64 Schur complement forms the cost blocks from
+// g), or with FP32 Schur rows (KKT_G_POS) only the knot-dependent 7x7 position block of Q_k:
+// the rest of G (the velocity diagonal, R, the zeros) depends on the cost weights only and is
+// written once per solve by gconst_kernel.
 #include "gpt_common.cuh"
 #include "gpt_dyn.cuh"
 #include "gpt_internal.h"
@@ -76,7 +77,7 @@ __device__ __forceinline__ void kkt_fetch(const float *xu, const float *goal, in
     v[3] = hl < 12 ? __ldg(goal + (size_t)6 * jj + hl) : 0.f;
 }
 
-template <bool FULL_G>
+template <int GMODE>
 __global__ void __launch_bounds__(32 * KKT_WARPS, 4) kkt_kernel(BatchView bv, ProblemParams P, const float *__restrict__ xu,
                                                            const float *__restrict__ goal,
                                                            const float *__restrict__ xs, float *__restrict__ G,
@@ -276,7 +277,7 @@ __global__ void __launch_bounds__(32 * KKT_WARPS, 4) kkt_kernel(BatchView bv, Pr
             }
             // ---- G_k = {Q_k, R_k}, g_k = {q_k, r_k}
             float *Gk = G + (size_t)G_STRIDE * j;
-            if constexpr (FULL_G) {
+            if constexpr (GMODE == KKT_G_FULL) {
                 for (int e = hl; e < G_STRIDE; e += 16) {
                     float v;
                     if (e < SS) {
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(32 * KKT_WARPS, 4) kkt_kernel(BatchView bv, Pr
                     }
                     Gk[e] = v;
                 }
-            } else if (hl < NQ) {
+            } else if (GMODE == KKT_G_POS && hl < NQ) {
 #pragma unroll
                 for (int i = 0; i < NQ; ++i) Gk[NS * i + hl] = sm.qv[0][i] * sm.qv[0][hl];
             }
@@ -295,12 +296,12 @@ __global__ void __launch_bounds__(32 * KKT_WARPS, 4) kkt_kernel(BatchView bv, Pr
                 g[(size_t)NX * j + e] = (e < NS) ? sm.qv[0][e] : P.r_cost * sm.u[e - NS];
             if (terminal) {
                 float *Gt = G + (size_t)G_STRIDE * (j + 1);
-                if constexpr (FULL_G) {
+                if constexpr (GMODE == KKT_G_FULL) {
                     for (int e = hl; e < SS; e += 16) {
                         const int i = e / NS, jq = e - NS * i;
                         Gt[e] = (i < NQ && jq < NQ) ? sm.qv[1][i] * sm.qv[1][jq] : ((i == jq) ? P.qd_cost : 0.f);
                     }
-                } else if (hl < NQ) {
+                } else if (GMODE == KKT_G_POS && hl < NQ) {
 #pragma unroll
                     for (int i = 0; i < NQ; ++i) Gt[NS * i + hl] = sm.qv[1][i] * sm.qv[1][hl];
                 }
@@ -339,17 +340,18 @@ __global__ void gconst_kernel(BatchView bv, float qd_cost, float r_cost, float *
 
 cudaError_t launch_kkt(const BatchView &bv, const ProblemParams &P, const float *xu, const float *goal,
                        const float *xs, float *G, float *C, float *g, float *c, int num_sms, cudaStream_t s,
-                       int ctas_per_sm, bool full_g)
+                       int ctas_per_sm, int g_mode)
 {
     if (bv.total_knots <= 0) return cudaSuccess;
     int warps = (bv.total_knots + 1) / 2;  // two knots per warp
     int blocks = (warps + KKT_WARPS - 1) / KKT_WARPS;
     const int cap = num_sms * ctas_per_sm;
     if (blocks > cap) blocks = cap;
-    if (full_g)
-        kkt_kernel<true><<<blocks, 32 * KKT_WARPS, 0, s>>>(bv, P, xu, goal, xs, G, C, g, c);
-    else
-        kkt_kernel<false><<<blocks, 32 * KKT_WARPS, 0, s>>>(bv, P, xu, goal, xs, G, C, g, c);
+    switch (g_mode) {
+    case KKT_G_FULL: kkt_kernel<KKT_G_FULL><<<blocks, 32 * KKT_WARPS, 0, s>>>(bv, P, xu, goal, xs, G, C, g, c); break;
+    case KKT_G_POS: kkt_kernel<KKT_G_POS><<<blocks, 32 * KKT_WARPS, 0, s>>>(bv, P, xu, goal, xs, G, C, g, c); break;
+    default: kkt_kernel<KKT_G_NONE><<<blocks, 32 * KKT_WARPS, 0, s>>>(bv, P, xu, goal, xs, G, C, g, c); break;
+    }
     return cudaGetLastError();
 }
 
