@@ -28,19 +28,8 @@
 
 namespace gpt {
 
-constexpr int ADJ_WARPS = 4;
+constexpr int ADJ_THREADS = 128;
 constexpr int ADJ_PART = 16;  // per-knot partials: qd 0..6, r 7..13, q_ee 14
-
-struct AdjWarpSmem {
-    float x[2][NS];      // x_k and x_{k+1}
-    float u[NC];
-    float goal[12];      // p*_k, p*_{k+1} (xyz + rpy)
-    float mu[2][NS];     // mu_z state parts of knots k, k+1
-    float muu[NC];
-    float d[2][NS];      // dz state parts of knots k, k+1
-    float du[NC];
-    float p[2][3], J[2][21];
-};
 
 __device__ __forceinline__ void adj_v(const float *J, const float *p, const float *t, float qee, float *v)
 {
@@ -62,148 +51,160 @@ __device__ __forceinline__ void adj_w(const float *a, const float *d, const floa
     for (int i = 0; i < NQ; ++i) w[i] = (float)((double)a[i] * (1.0 - vd) - (double)d[i] * av);
 }
 
-__global__ void __launch_bounds__(32 * ADJ_WARPS)
+// One thread per knot (a warp per knot had one lane do the forward kinematics: 164 -> 16 us at 512 x 128).
+__global__ void __launch_bounds__(ADJ_THREADS)
     adjoint_grad_kernel(BatchView bv, ProblemParams P, const float *__restrict__ xu, const float *__restrict__ goal,
                         const float *__restrict__ dz, const float *__restrict__ mu, float *__restrict__ grad_goal,
                         float *__restrict__ part)
 {
-    __shared__ AdjWarpSmem smem_all[ADJ_WARPS];
-    const int lane = threadIdx.x & 31;
-    AdjWarpSmem &sm = smem_all[threadIdx.x >> 5];
-    const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int j = bv.j0 + gw; j < bv.j0 + bv.total_knots; j += nw) {
+    const int jend = bv.j0 + bv.total_knots;
+    for (int j = bv.j0 + blockIdx.x * blockDim.x + threadIdx.x; j < jend; j += gridDim.x * blockDim.x) {
         const int b = bv.inst(j);
         if (!bv.active(b)) continue;
         const int N = bv.N(b), k = j - bv.off(b);
-        float *pk = part + (size_t)ADJ_PART * j;
         if (k == N - 1) continue;  // the terminal knot is handled with knot N-2
         const bool terminal = (k == N - 2);
-        // ---- stage x_k, u_k, x_{k+1}, goals, mu and dz of knots k, k+1
-        for (int i = lane; i < NX + NS; i += 32) {
-            const size_t o = (size_t)NX * j + i;
-            if (i < NS) {
-                sm.x[0][i] = xu[o];
-                sm.mu[0][i] = mu[o];
-                sm.d[0][i] = dz[o];
-            } else if (i < NX) {
-                sm.u[i - NS] = xu[o];
-                sm.muu[i - NS] = mu[o];
-                sm.du[i - NS] = dz[o];
-            } else {
-                sm.x[1][i - NX] = xu[o];
-                sm.mu[1][i - NX] = mu[o];
-                sm.d[1][i - NX] = dz[o];
-            }
+        const float *x0 = xu + (size_t)NX * j, *d0 = dz + (size_t)NX * j, *m0 = mu + (size_t)NX * j;
+        const float *gl = goal + (size_t)6 * j;
+        const float qee = P.q_ee;
+        float q[NQ], mq[NQ], dq[NQ], p[3], Jac[3 * NQ], v[NQ], w[NQ], e[3];
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+            q[i] = x0[i];
+            mq[i] = m0[i];
+            dq[i] = d0[i];
         }
-        if (lane < 12) sm.goal[lane] = goal[(size_t)6 * j + lane];
-        __syncwarp();
-        // ---- forward kinematics and position Jacobian: lane 0 at x_k, lane 1 at x_{k+1}
-        if (lane == 0 || (lane == 1 && terminal && !P.ref_terminal)) {
+        {
             JointTrig t;
-            joint_trig(sm.x[lane], t);
-            fk_lane<true>(t, sm.p[lane], sm.J[lane]);
+            joint_trig(q, t);
+            fk_lane<true>(t, p, Jac);
         }
-        __syncwarp();
-        if (lane == 0) {
-            const float qee = P.q_ee;
-            float v[NQ], w[NQ], e[3];
-            for (int dd = 0; dd < 3; ++dd) e[dd] = sm.p[0][dd] - sm.goal[dd];
-            adj_v(sm.J[0], sm.p[0], sm.goal, qee, v);
-            adj_w(sm.mu[0], sm.d[0], v, w);
-            double gq = 0.0;                                  // d l / d q_ee
-            float gg_next[3] = {0.f, 0.f, 0.f};               // d l / d p*_{k+1} (terminal, spec mode)
-            double qd_part[NQ], r_part[NC];
 #pragma unroll
-            for (int i = 0; i < NQ; ++i)
-                qd_part[i] = (double)sm.mu[0][NQ + i] * ((double)sm.x[0][NQ + i] - (double)sm.d[0][NQ + i]);
+        for (int dd = 0; dd < 3; ++dd) e[dd] = p[dd] - gl[dd];
+        adj_v(Jac, p, gl, qee, v);
+        adj_w(mq, dq, v, w);
+        double gq = 0.0;                     // d l / d q_ee
+        float gg_next[3] = {0.f, 0.f, 0.f};  // d l / d p*_{k+1} (terminal, spec mode)
+        double qd_part[NQ];
 #pragma unroll
-            for (int i = 0; i < NC; ++i) r_part[i] = (double)sm.muu[i] * ((double)sm.u[i] - (double)sm.du[i]);
-            if (terminal) {
-                // terminal cost block (knot N-1)
-                const int which = P.ref_terminal ? 0 : 1;
-                const float *xt = P.ref_terminal ? sm.x[0] : sm.x[1];
-                float tt[3];
-                if (P.ref_terminal) {
-                    const float a0 = v[0];
-                    tt[0] = a0 * a0;
-                    tt[1] = a0 * v[1];
-                    tt[2] = a0 * v[2];
-                } else {
-                    tt[0] = sm.goal[6];
-                    tt[1] = sm.goal[7];
-                    tt[2] = sm.goal[8];
-                }
-                float vt[NQ], wt[NQ];
-                adj_v(sm.J[which], sm.p[which], tt, qee, vt);
-                adj_w(sm.mu[1], sm.d[1], vt, wt);
-                // d l / d target = -q_ee J_t w_t
-                float gt[3];
-                for (int dd = 0; dd < 3; ++dd) {
-                    double a = 0.0;
+        for (int i = 0; i < NQ; ++i) qd_part[i] = (double)m0[NQ + i] * ((double)x0[NQ + i] - (double)d0[NQ + i]);
+        if (terminal) {
+            // terminal cost block (knot N-1)
+            const float *x1 = x0 + NX, *d1 = d0 + NX, *m1 = m0 + NX;
+            const float *xt = P.ref_terminal ? x0 : x1;
+            float tt[3], pt[3], Jt[3 * NQ], vt[NQ], wt[NQ], md[NQ], ddq[NQ];
+            if (P.ref_terminal) {
+                const float a0 = v[0];
+                tt[0] = a0 * a0;
+                tt[1] = a0 * v[1];
+                tt[2] = a0 * v[2];
 #pragma unroll
-                    for (int i = 0; i < NQ; ++i) a += (double)sm.J[which][3 * i + dd] * wt[i];
-                    gt[dd] = (float)(-(double)qee * a);
-                }
-                // direct q_ee dependence of v_t = q_ee J_t^T (p_t - t)
-                for (int i = 0; i < NQ; ++i) {
-                    double a = 0.0;
-                    for (int dd = 0; dd < 3; ++dd)
-                        a += (double)sm.J[which][3 * i + dd] * ((double)sm.p[which][dd] - (double)tt[dd]);
-                    gq += (double)wt[i] * a;
-                }
-                if (P.ref_terminal) {
-                    // t = (a0^2, a0 a1, a0 a2) with a = v_{N-2}: the target's adjoint flows into w_{N-2}
-                    w[0] += 2.f * v[0] * gt[0] + v[1] * gt[1] + v[2] * gt[2];
-                    w[1] += v[0] * gt[1];
-                    w[2] += v[0] * gt[2];
-                } else {
-                    for (int dd = 0; dd < 3; ++dd) gg_next[dd] = gt[dd];
-                }
-                // terminal velocity cost qd .* qdot_t
+                for (int i = 0; i < 3; ++i) pt[i] = p[i];
 #pragma unroll
-                for (int i = 0; i < NQ; ++i)
-                    qd_part[i] += (double)sm.mu[1][NQ + i] * ((double)xt[NQ + i] - (double)sm.d[1][NQ + i]);
+                for (int i = 0; i < 3 * NQ; ++i) Jt[i] = Jac[i];
+            } else {
+                tt[0] = gl[6];
+                tt[1] = gl[7];
+                tt[2] = gl[8];
+                float q1[NQ];
+#pragma unroll
+                for (int i = 0; i < NQ; ++i) q1[i] = x1[i];
+                JointTrig t;
+                joint_trig(q1, t);
+                fk_lane<true>(t, pt, Jt);
             }
-            // knot k: d l / d p*_k = -q_ee J_k w_k and the q_ee term w_k^T J_k^T e_k
+#pragma unroll
+            for (int i = 0; i < NQ; ++i) {
+                md[i] = m1[i];
+                ddq[i] = d1[i];
+            }
+            adj_v(Jt, pt, tt, qee, vt);
+            adj_w(md, ddq, vt, wt);
+            // d l / d target = -q_ee J_t w_t
+            float gt[3];
+#pragma unroll
             for (int dd = 0; dd < 3; ++dd) {
                 double a = 0.0;
 #pragma unroll
-                for (int i = 0; i < NQ; ++i) a += (double)sm.J[0][3 * i + dd] * w[i];
-                grad_goal[(size_t)6 * j + dd] = (float)(-(double)qee * a);
+                for (int i = 0; i < NQ; ++i) a += (double)Jt[3 * i + dd] * wt[i];
+                gt[dd] = (float)(-(double)qee * a);
             }
+            // direct q_ee dependence of v_t = q_ee J_t^T (p_t - t)
+#pragma unroll
             for (int i = 0; i < NQ; ++i) {
                 double a = 0.0;
-                for (int dd = 0; dd < 3; ++dd) a += (double)sm.J[0][3 * i + dd] * e[dd];
-                gq += (double)w[i] * a;
-            }
-            for (int dd = 3; dd < 6; ++dd) grad_goal[(size_t)6 * j + dd] = 0.f;
-            if (terminal) {
-                for (int dd = 0; dd < 3; ++dd) grad_goal[(size_t)6 * (j + 1) + dd] = gg_next[dd];
-                for (int dd = 3; dd < 6; ++dd) grad_goal[(size_t)6 * (j + 1) + dd] = 0.f;
-            }
 #pragma unroll
-            for (int i = 0; i < NQ; ++i) pk[i] = (float)qd_part[i];
+                for (int dd = 0; dd < 3; ++dd) a += (double)Jt[3 * i + dd] * ((double)pt[dd] - (double)tt[dd]);
+                gq += (double)wt[i] * a;
+            }
+            if (P.ref_terminal) {
+                // t = (a0^2, a0 a1, a0 a2) with a = v_{N-2}: the target's adjoint flows into w_{N-2}
+                w[0] += 2.f * v[0] * gt[0] + v[1] * gt[1] + v[2] * gt[2];
+                w[1] += v[0] * gt[1];
+                w[2] += v[0] * gt[2];
+            } else {
 #pragma unroll
-            for (int i = 0; i < NC; ++i) pk[NQ + i] = (float)r_part[i];
-            pk[14] = (float)gq;
+                for (int dd = 0; dd < 3; ++dd) gg_next[dd] = gt[dd];
+            }
+            // terminal velocity cost qd .* qdot_t
+#pragma unroll
+            for (int i = 0; i < NQ; ++i)
+                qd_part[i] += (double)m1[NQ + i] * ((double)xt[NQ + i] - (double)d1[NQ + i]);
         }
-        __syncwarp();
+        // knot k: d l / d p*_k = -q_ee J_k w_k and the q_ee term w_k^T J_k^T e_k
+        float *gk = grad_goal + (size_t)6 * j;
+#pragma unroll
+        for (int dd = 0; dd < 3; ++dd) {
+            double a = 0.0;
+#pragma unroll
+            for (int i = 0; i < NQ; ++i) a += (double)Jac[3 * i + dd] * w[i];
+            gk[dd] = (float)(-(double)qee * a);
+            gk[3 + dd] = 0.f;
+        }
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+            double a = 0.0;
+#pragma unroll
+            for (int dd = 0; dd < 3; ++dd) a += (double)Jac[3 * i + dd] * e[dd];
+            gq += (double)w[i] * a;
+        }
+        if (terminal) {
+#pragma unroll
+            for (int dd = 0; dd < 3; ++dd) {
+                gk[6 + dd] = gg_next[dd];
+                gk[9 + dd] = 0.f;
+            }
+        }
+        float *pk = part + (size_t)ADJ_PART * j;
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) {
+            pk[i] = (float)qd_part[i];
+            pk[NQ + i] = (float)((double)m0[NS + i] * ((double)x0[NS + i] - (double)d0[NS + i]));
+        }
+        pk[14] = (float)gq;
     }
 }
 
-// per instance: fixed-order FP64 sums of the per-knot partials (knots 0..N-2)
-// (wacc: added to wacc[15 b + t] instead)
-__global__ void adjoint_reduce_kernel(BatchView bv, const float *__restrict__ part, float *__restrict__ grad_qd,
-                                      float *__restrict__ grad_r, float *__restrict__ grad_qee, float *__restrict__ wacc)
+// per instance: fixed-order FP64 sums of the per-knot partials (knots 0..N-2): thread (g, t) sums component t of the
+// knots g, g + RED_GROUPS, ...; the groups' sums are added in order (wacc: added to wacc[15 b + t] instead).  One
+// thread per component walked the horizon alone: 40 -> 6 us at 512 x 128, 30 -> 5 us for 33 instances of up to 96 knots.
+constexpr int RED_GROUPS = 16;
+__global__ void __launch_bounds__(ADJ_PART *RED_GROUPS)
+    adjoint_reduce_kernel(BatchView bv, const float *__restrict__ part, float *__restrict__ grad_qd,
+                          float *__restrict__ grad_r, float *__restrict__ grad_qee, float *__restrict__ wacc)
 {
+    __shared__ double sums[RED_GROUPS][ADJ_PART];
     const int b = bv.b0 + (int)blockIdx.x;
-    if (b >= bv.b0 + bv.B || !bv.active(b)) return;
-    const int t = threadIdx.x;  // 0..14
-    if (t >= 15) return;
+    if (!bv.active(b)) return;
+    const int t = threadIdx.x % ADJ_PART, g = threadIdx.x / ADJ_PART;
     const int N = bv.N(b), kb = bv.off(b);
     double a = 0.0;
-    for (int k = 0; k < N - 1; ++k) a += (double)part[(size_t)ADJ_PART * (kb + k) + t];
+    if (t < 15)
+        for (int k = g; k < N - 1; k += RED_GROUPS) a += (double)part[(size_t)ADJ_PART * (kb + k) + t];
+    sums[g][t] = a;
+    __syncthreads();
+    if (g > 0 || t >= 15) return;
+    for (int i = 1; i < RED_GROUPS; ++i) a += sums[i][t];
     if (wacc) wacc[(size_t)15 * b + t] += (float)a;
     else if (t < NQ) grad_qd[(size_t)NQ * b + t] = (float)a;
     else if (t < NQ + NC) grad_r[(size_t)NC * b + t - NQ] = (float)a;
@@ -223,12 +224,14 @@ cudaError_t launch_adjoint_grad(const BatchView &bv, const ProblemParams &P, con
                                 float *grad_r, float *grad_qee, int num_sms, cudaStream_t s, float *wacc)
 {
     if (bv.total_knots <= 0) return cudaSuccess;
-    int blocks = (bv.total_knots + ADJ_WARPS - 1) / ADJ_WARPS;
+    // few knots: a warp per block, so that they spread over the SMs
+    const int threads = bv.total_knots < num_sms * ADJ_THREADS ? 32 : ADJ_THREADS;
+    int blocks = (bv.total_knots + threads - 1) / threads;
     if (blocks > num_sms * 16) blocks = num_sms * 16;
-    adjoint_grad_kernel<<<blocks, 32 * ADJ_WARPS, 0, s>>>(bv, P, xu, goal, dz, mu, grad_goal, part);
+    adjoint_grad_kernel<<<blocks, threads, 0, s>>>(bv, P, xu, goal, dz, mu, grad_goal, part);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    adjoint_reduce_kernel<<<bv.B, 32, 0, s>>>(bv, part, grad_qd, grad_r, grad_qee, wacc);
+    adjoint_reduce_kernel<<<bv.B, ADJ_PART * RED_GROUPS, 0, s>>>(bv, part, grad_qd, grad_r, grad_qee, wacc);
     return cudaGetLastError();
 }
 
