@@ -150,6 +150,9 @@ struct gpt_handle {
     int *h_trk_rows = nullptr;
     TrackInst *h_trk_inst = nullptr;
     cudaStream_t cap_stream = nullptr, body_stream = nullptr;
+    // the plant simulation of a control update, beside the update's solve
+    cudaStream_t sim_stream = nullptr;
+    cudaEvent_t ev_sim_fork = nullptr, ev_sim_join = nullptr;
     // the part-batch branches of a graph iteration (sqp_graph >= 2): streams 1.. and their events
     cudaStream_t branch_stream[MAX_BRANCHES] = {};
     cudaEvent_t ev_fork = nullptr, ev_join[MAX_BRANCHES] = {};
@@ -396,6 +399,9 @@ gpt_status gpt_create(const gpt_problem_config *pc, const gpt_solver_config *sc,
     ALLOC(trk_kloss, T);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->cap_stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->body_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->sim_stream, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_sim_fork, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_sim_join, cudaEventDisableTiming);
     for (int i = 1; i < MAX_BRANCHES; ++i) {
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->branch_stream[i], cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->ev_join[i], cudaEventDisableTiming);
@@ -472,6 +478,9 @@ gpt_status gpt_destroy(gpt_handle *h)
     cudaFreeHost(h->h_knot_off); cudaFreeHost(h->h_knot_inst);
     if (h->cap_stream) cudaStreamDestroy(h->cap_stream);
     if (h->body_stream) cudaStreamDestroy(h->body_stream);
+    if (h->sim_stream) cudaStreamDestroy(h->sim_stream);
+    if (h->ev_sim_fork) cudaEventDestroy(h->ev_sim_fork);
+    if (h->ev_sim_join) cudaEventDestroy(h->ev_sim_join);
     for (int i = 1; i < MAX_BRANCHES; ++i) {
         if (h->branch_stream[i]) cudaStreamDestroy(h->branch_stream[i]);
         if (h->ev_join[i]) cudaEventDestroy(h->ev_join[i]);
@@ -1454,6 +1463,35 @@ static gpt_status enqueue_track_adjoint(gpt_handle *h, const SqpPlan &pl, float 
     return GPT_OK;
 }
 
+// Work on the handle's simulation stream between begin() and end(): it starts after the work enqueued on s so far, and s
+// goes on after it.  An open fork is joined when the scope ends, so that an early return leaves no work that the caller's
+// stream does not wait for.
+struct SimFork {
+    gpt_handle *h;
+    cudaStream_t s;
+    bool open = false;
+    SimFork(gpt_handle *h_, cudaStream_t s_) : h(h_), s(s_) {}
+    cudaError_t begin()
+    {
+        cudaError_t e = cudaEventRecord(h->ev_sim_fork, s);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(h->sim_stream, h->ev_sim_fork, 0);
+        open = e == cudaSuccess;
+        return e;
+    }
+    cudaError_t end()
+    {
+        open = false;
+        const cudaError_t e = cudaEventRecord(h->ev_sim_join, h->sim_stream);
+        return e == cudaSuccess ? cudaStreamWaitEvent(s, h->ev_sim_join, 0) : e;
+    }
+    ~SimFork()
+    {
+        if (open) end();
+    }
+    SimFork(const SimFork &) = delete;
+    SimFork &operator=(const SimFork &) = delete;
+};
+
 // gpt_track_batched, and with d_wgrad non-null gpt_track_batched_adjoint
 static gpt_status track_impl(gpt_handle *h, uint32_t B, const uint32_t *h_N, const uint32_t *h_S,
                              const float *d_eePos_traj, const float *d_xu_traj, float *d_xs,
@@ -1513,16 +1551,24 @@ static gpt_status track_impl(gpt_handle *h, uint32_t B, const uint32_t *h_N, con
                                         1, ns, s));
         }
     }
+    // An update's plant simulation needs the state and the previous update's controls only, so it runs on a stream of
+    // its own beside the solve (it is a chain of plant steps, 80 us for 50 of them, on one warp per four
+    // instances); the update's shift waits for both.
+    SimFork fork(h, s);
     for (uint32_t u = 0; u < n_updates; ++u) {
         GPT_CUDA(launch_track_prep(bv, h->trk_rows, h->trk_clk, tc.rho_reset, 0, s));
+        GPT_CUDA(launch_track_clock(h->trk_clk, tp, s));
+        GPT_CUDA(fork.begin());
+        GPT_CUDA(launch_track_sim(bv, h->trk_rows, h->trk_clk, tp, d_xs, h->trk_xu_old, h->sim_stream));
         const gpt_status st = solve_on_workspace(h, plan, s);
         if (st != GPT_OK) return st;
         if (d_wgrad) {
             const gpt_status sa = enqueue_track_adjoint(h, plan, d_wgrad, d_loss, s);
             if (sa != GPT_OK) return sa;
         }
-        GPT_CUDA(launch_track_tail(bv, h->trk_rows, h->trk_clk, tp, d_eePos_traj, d_xu_traj, d_xs, h->gxu,
-                                   h->trk_xu_old, h->ggoal, h->glam, h->adj_h, d_err, h->trk_inst, d_log, log_cap, s));
+        GPT_CUDA(fork.end());
+        GPT_CUDA(launch_track_post(bv, h->trk_rows, h->trk_clk, d_eePos_traj, d_xu_traj, d_xs, h->gxu, h->trk_xu_old,
+                                   h->ggoal, h->glam, h->adj_h, d_err, h->trk_inst, d_log, log_cap, s));
     }
     GPT_CUDA(launch_track_final(bv, d_xs, h->ggoal, h->trk_inst, s));
     GPT_CUDA(cudaMemcpyAsync(h->h_trk_inst, h->trk_inst, sizeof(TrackInst) * B, cudaMemcpyDeviceToHost, s));

@@ -133,10 +133,14 @@ cudaError_t launch_track_start(const BatchView &bv, const int *rows, const float
                                float rho0, int reset_xu_only, int num_sms, cudaStream_t s);
 cudaError_t launch_track_prep(const BatchView &bv, const int *rows, const TrackClock *clk, float rho_reset,
                               int all_live, cudaStream_t s);
-cudaError_t launch_track_tail(const BatchView &bv, const int *rows, TrackClock *clk, const TrackParams &tp,
-                              const float *eePos_traj, const float *xu_traj, float *xs, float *xu, float *xu_old,
-                              float *goal, float *lambda, float *tmp, float *errors, TrackInst *inst,
-                              uint32_t *iters_log, uint32_t log_cap, cudaStream_t s);
+// an update's clock (read by prep before it and by the rest after it), plant simulation, and bookkeeping and shift
+cudaError_t launch_track_clock(TrackClock *clk, const TrackParams &tp, cudaStream_t s);
+cudaError_t launch_track_sim(const BatchView &bv, const int *rows, const TrackClock *clk, const TrackParams &tp,
+                             float *xs, const float *xu_old, cudaStream_t s);
+cudaError_t launch_track_post(const BatchView &bv, const int *rows, const TrackClock *clk, const float *eePos_traj,
+                              const float *xu_traj, const float *xs, float *xu, float *xu_old, float *goal,
+                              float *lambda, float *tmp, float *errors, TrackInst *inst, uint32_t *iters_log,
+                              uint32_t log_cap, cudaStream_t s);
 cudaError_t launch_track_final(const BatchView &bv, const float *xs, const float *goal, TrackInst *inst, cudaStream_t s);
 // the adjoint of each update's solve (gpt_track_batched_adjoint): begin saves the per-solve state and
 // marks the instances that track this update active; loss_grad writes h = dl/d(dz) = -dl/dxu+ of the

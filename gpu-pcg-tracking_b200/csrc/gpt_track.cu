@@ -263,19 +263,26 @@ cudaError_t launch_track_prep(const BatchView &bv, const int *rows, const TrackC
     return cudaGetLastError();
 }
 
-cudaError_t launch_track_tail(const BatchView &bv, const int *rows, TrackClock *clk, const TrackParams &tp,
-                              const float *eePos_traj, const float *xu_traj, float *xs, float *xu, float *xu_old,
-                              float *goal, float *lambda, float *tmp, float *errors, TrackInst *inst,
-                              uint32_t *iters_log, uint32_t log_cap, cudaStream_t s)
+cudaError_t launch_track_clock(TrackClock *clk, const TrackParams &tp, cudaStream_t s)
 {
     track_clock_kernel<<<1, 1, 0, s>>>(clk, tp);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_track_sim(const BatchView &bv, const int *rows, const TrackClock *clk, const TrackParams &tp,
+                             float *xs, const float *xu_old, cudaStream_t s)
+{
     // one warp (4 instances) per CTA: the kernel is a dependent chain per instance, so the
     // instances spread over as many SMs as possible
     track_sim_kernel<<<(bv.B + 3) / 4, 32, 0, s>>>(bv, rows, clk, tp, xs, xu_old);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    return cudaGetLastError();
+}
+
+cudaError_t launch_track_post(const BatchView &bv, const int *rows, const TrackClock *clk, const float *eePos_traj,
+                              const float *xu_traj, const float *xs, float *xu, float *xu_old, float *goal,
+                              float *lambda, float *tmp, float *errors, TrackInst *inst, uint32_t *iters_log,
+                              uint32_t log_cap, cudaStream_t s)
+{
     track_post_kernel<<<bv.B, POST_THREADS, 0, s>>>(bv, rows, clk, eePos_traj, xu_traj, xs, xu, xu_old, goal, lambda,
                                                     tmp, errors, inst, iters_log, log_cap);
     return cudaGetLastError();
@@ -290,7 +297,8 @@ cudaError_t launch_track_final(const BatchView &bv, const float *xs, const float
 // ---- the adjoint of each update's solve (gpt_track_batched_adjoint; no reference counterpart)
 
 // Saves every instance's per-solve state (the adjoint's KKT, Schur and PCG launches reuse the
-// solve's kernels, which count into it) and marks the instances that track this update active.
+// solve's kernels, which count into it) and marks the instances that track this update active (the
+// clock has been advanced to the update's end: its offset at the start counts).
 __global__ void track_adj_begin_kernel(BatchView bv, const int *__restrict__ rows, const TrackClock *__restrict__ clk,
                                        InstState *__restrict__ bak)
 {
@@ -298,7 +306,7 @@ __global__ void track_adj_begin_kernel(BatchView bv, const int *__restrict__ row
     if (b >= bv.B) return;
     InstState &s = bv.st[b];
     bak[b] = s;
-    s.active = clk->traj_offset < (uint32_t)(rows[b + 1] - rows[b]) ? 1u : 0u;
+    s.active = clk->start_offset < (uint32_t)(rows[b + 1] - rows[b]) ? 1u : 0u;
     s.exit_flags = 0u;
     s.pcg_maxiter_count = 0u;
 }
