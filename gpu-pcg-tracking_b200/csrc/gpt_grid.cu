@@ -14,6 +14,7 @@
 // states (14 floats) are both accepted.
 #include "gpt_common.cuh"
 #include "gpt_dyn.cuh"
+#include "gpt_fdlane.cuh"
 #include "gpt_internal.h"
 
 namespace gpt {
@@ -153,9 +154,52 @@ __global__ void __launch_bounds__(32 * FDG_WARPS)
     }
 }
 
+// The same with one row per lane (gpt_fdlane.cuh), eight warps per SM (255 registers a thread, 26 KB of shared memory a
+// warp).  200,003 rows: 138 us against the half-warp form's 437, both cut by the issue of the tangent passes and their
+// latency (the rows' 685 bytes would take 21 us); two warps per CTA fill the last wave best (four 140, eight 154).
+constexpr int FDGL_WARPS = 2;
+
+__global__ void __launch_bounds__(32 * FDGL_WARPS, 8 / FDGL_WARPS)
+    fd_grad_lane_kernel(uint32_t n, const float *__restrict__ xu, uint32_t stride, float *__restrict__ qdd_out,
+                        float *__restrict__ df_out)
+{
+    extern __shared__ float4 fdgl_dyn_smem[];
+    const int lane = threadIdx.x & 31;
+    FdLaneSmem &sm = reinterpret_cast<FdLaneSmem *>(fdgl_dyn_smem)[threadIdx.x >> 5];
+    const size_t i0 = (size_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
+    const bool valid = i0 + lane < n;  // lanes past the end follow the last row and store nothing
+    const uint32_t mask = __ballot_sync(0xffffffffu, valid);
+    const float *x = xu + (size_t)stride * (valid ? i0 + lane : n - 1);
+    float q[NQ], qd[NQ], u[NC], qdd[NQ];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+        q[i] = x[i];
+        qd[i] = x[NQ + i];
+        u[i] = x[NS + i];
+    }
+    JointTrig t;
+    joint_trig(q, t);
+    fd_gradient_lane(t, qd, u, qdd, sm, lane, [&](int col, const float (&v)[NQ]) {
+        store_rows<NQ>(sm.out, v, df_out + NQ * NX * i0 + NQ * col, NQ * NX, mask, lane);
+    });
+    store_rows<NQ>(sm.out, qdd, qdd_out + NQ * i0, NQ, mask, lane);
+}
+
 cudaError_t launch_fd_grad(uint32_t n, const float *xu, uint32_t stride, float *qdd, float *df, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
+    // One row per lane from FDGL_MIN rows on: up to four warps per SM (18,944 rows) that form takes 21 us whatever the
+    // number of rows, the half-warp form 2.5 us per 1,000 rows beyond its own 4 (8,000 rows 23.7 against 21.2 us, 16,000
+    // rows 40.3 against 21.2)
+    constexpr uint32_t FDGL_MIN = 8192;
+    if (n >= FDGL_MIN) {
+        constexpr int per = 32 * FDGL_WARPS;
+        const size_t smem = sizeof(FdLaneSmem) * FDGL_WARPS;
+        const cudaError_t e = ensure_func_attrs((const void *)fd_grad_lane_kernel, smem);
+        if (e != cudaSuccess) return e;
+        fd_grad_lane_kernel<<<(unsigned)(((size_t)n + per - 1) / per), per, smem, s>>>(n, xu, stride, qdd, df);
+        return cudaGetLastError();
+    }
     fd_grad_kernel<<<(unsigned)(((size_t)n * 16 + 32 * FDG_WARPS - 1) / (32 * FDG_WARPS)), 32 * FDG_WARPS, 0, s>>>(
         n, xu, stride, qdd, df);
     return cudaGetLastError();

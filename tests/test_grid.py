@@ -98,3 +98,35 @@ def test_forward_dynamics_gradient_matches_oracle(gpt, oracle, golden):
         for b in range(3):
             blk = slice(49 * b, 49 * (b + 1))
             assert np.abs(df[k, blk] - wdf[blk]).max() <= 1e-4 * max(1e-3, np.abs(wdf[blk]).max()), (k, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,stride", [(8191, 21), (8192, 21), (8193, 22), (8192 + 63, 24), (18944 + 65, 21), (40001, 21)])
+def test_forward_dynamics_gradient_by_row_count(gpt, oracle, golden, n, stride):
+    """Both forms of the gradient (a half-warp per row below 8192 rows, a lane per row from there on) against the FP64
+    oracle at the edges of their ranges, with the tolerances of the test above; a row of NaN stays alone, and nothing is
+    written past the last row."""
+    tr = np.concatenate([golden["traj_0_1"], golden["traj_3_4"]])
+    rng = np.random.default_rng(n)
+    rows = tr[rng.integers(0, len(tr), n), :21] + rng.uniform(-0.1, 0.1, (n, 21)).astype(np.float32)
+    bad = n // 2
+    x = np.zeros((n, stride), np.float32)
+    x[:, :21] = rows
+    x[bad, 3] = np.nan
+    xu = dev(x)
+    qdd_t, df_t = (torch.full((n + 3, w), 7.0, device="cuda") for w in (7, 147))
+    gpt._check(gpt.lib().gpt_forward_dynamics_gradient(n, gpt._ptr(xu), stride, gpt._ptr(qdd_t), gpt._ptr(df_t),
+                                                       gpt._stream(None)))
+    torch.cuda.synchronize()
+    qdd, df = qdd_t.cpu().numpy(), df_t.cpu().numpy()
+    assert (qdd[n:] == 7.0).all() and (df[n:] == 7.0).all()
+    ok = np.arange(n) != bad
+    assert np.isfinite(qdd[:n][ok]).all() and np.isfinite(df[:n][ok]).all() and np.isnan(qdd[bad]).all()
+    check = np.unique(np.concatenate([np.arange(3), np.arange(n - 40, n), [bad - 1, bad + 1], rng.integers(0, n, 40)]))
+    for k in check[check != bad]:
+        row = x[k].astype(np.float64)
+        wq, wdf = oracle.fd_grad(row[:7], row[7:14], row[14:21])
+        assert np.abs(qdd[k] - wq).max() <= 1e-5 * max(1.0, np.abs(wq).max()), k
+        for b in range(3):
+            blk = slice(49 * b, 49 * (b + 1))
+            assert np.abs(df[k, blk] - wdf[blk]).max() <= 1e-4 * max(1e-3, np.abs(wdf[blk]).max()), (k, b)
