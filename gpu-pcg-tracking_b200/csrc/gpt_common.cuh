@@ -60,6 +60,8 @@ struct BatchView {
     // the partitioned PCG's warps per instance, fixed by the whole batch so that its parts give the same bits
     // (0: by this view)
     int part_warps = 0;
+    // KKT formation with one knot per lane (a choice for the whole batch too)
+    bool kkt_lane = false;
 
     __device__ __forceinline__ int inst(int j) const { return knot_inst ? knot_inst[j] : 0; }
     __device__ __forceinline__ int off(int b) const { return knot_off ? knot_off[b] : 0; }

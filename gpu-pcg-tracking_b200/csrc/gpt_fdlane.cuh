@@ -1,5 +1,5 @@
 // gpt_fdlane.cuh -- forward dynamics and its gradient with one state per lane (32 states per warp): the throughput
-// form of the half-warp evaluation in gpt_grid.cu, which gives 16 lanes a state and has every lane
+// form of the half-warp evaluation in gpt_kkt.cu and gpt_grid.cu, which gives 16 lanes a state and has every lane
 // repeat the value pass beside its tangent.  Here the value pass runs once per state and each tangent only through the
 // links it reaches (direction j leaves the links before j at rest), about 600 instructions of a warp per state
 // against 2150.  A warp takes some 20 us whatever the number of states, so the half-warp form stays the better one for
@@ -19,7 +19,7 @@ constexpr int FL_V = 0, FL_IV = 6 * model::NJ, FL_XA = 12 * model::NJ, FL_F = 16
 struct FdLaneSmem {
     float base[FL_N][32];  // per link: v (6), I v (6), X a (entries 0, 1, 3, 4), accumulated f (the same entries)
     float Minv[CC][32];
-    float out[NS * 33];    // a block of output rows on its way to memory
+    float out[NS * 34];    // a block of output rows on its way to memory (store_rows)
 };
 
 // ---- two FP32 values per operation (fma.rn.f32x2): the mass matrix's columns 2p, 2p + 1 and the tangents of q_d and
@@ -360,6 +360,12 @@ __device__ __forceinline__ void fl_tangent_bwd(const JointTrig &t, int d, f2 (&d
         fl_tangent_bwd<J - 1>(t, d, df, sm, lane);
     }
 }
+// a block of df/du's columns: d/dq, d/dqd, d/du
+template <int I>
+struct FdBlock {
+    static constexpr int block = I;
+};
+
 // The CTA's warps take the directions together (the barrier): the loop's code then comes from the instruction cache once
 // for the warps of a scheduler instead of once for each, which is what bounds the kernel.
 template <class Emit>
@@ -382,13 +388,13 @@ __device__ __forceinline__ void fl_directions(const JointTrig &t, const float (&
             for (int k = 0; k < NQ; ++k) acc = fma2(du2(sm.Minv[r + NQ * k][lane]), df[k][2], acc);
             un2(neg2(acc), lo[r], hi[r]);
         }
-        emit(d, lo);
-        emit(NQ + d, hi);
+        emit(FdBlock<0>(), d, lo);
+        emit(FdBlock<1>(), d, hi);
     }
 }
 
 // qdd = M^{-1} (u - c) and the columns of df/du = [-M^{-1} dID/dq, -M^{-1} dID/dqd, M^{-1}] at (q, qd, u), each handed to
-// emit(column, values[7]) by every lane at the same time
+// emit(FdBlock<i>(), column of the block, values[7]) by every lane at the same time
 template <class Emit>
 __device__ __forceinline__ void fd_gradient_lane(const JointTrig &t, const float (&qd)[NQ], const float (&u)[NC],
                                                  float (&qdd)[NQ], FdLaneSmem &sm, int lane, Emit emit)
@@ -450,25 +456,30 @@ __device__ __forceinline__ void fd_gradient_lane(const JointTrig &t, const float
         float col[NQ];
 #pragma unroll
         for (int r = 0; r < NQ; ++r) col[r] = sm.Minv[r + NQ * j][lane];
-        emit(2 * NQ + j, col);
+        emit(FdBlock<2>(), j, col);
     }
 }
 
-// Store R values per lane (v[0 .. R-1] of state i = lane) as R consecutive floats at dst + stride i for the lanes in
-// mask, through shared memory so that the stores of neighbouring lanes are contiguous; every lane calls it
-template <int R>
-__device__ __forceinline__ void store_rows(float (&buf)[NS * 33], const float (&v)[R], float *dst, int stride, uint32_t mask,
-                                           int lane)
+// Store R values per lane (v[0 .. R-1] of state i = lane) as R consecutive floats at dst + STRIDE i for the lanes in
+// mask; every lane calls it.  Through shared memory, 32 / R states by R lanes at a time: a store then covers that many
+// contiguous runs, its addresses differ from the last one's by a constant, and neither side has bank conflicts.
+template <int R, int STRIDE>
+__device__ __forceinline__ void store_rows(float (&buf)[NS * 34], const float (&v)[R], float *dst, uint32_t mask, int lane)
 {
-    static_assert(R <= NS, "the buffer's rows");
+    constexpr int K = 32 / R, PITCH = 32 + K;
+    static_assert(R * PITCH <= NS * 34 && 32 % K == 0, "the buffer");
     __syncwarp();
 #pragma unroll
-    for (int r = 0; r < R; ++r) buf[33 * r + lane] = v[r];
+    for (int r = 0; r < R; ++r) buf[PITCH * r + lane] = v[r];
     __syncwarp();
+    const int k = lane / R, r = lane - R * k;
+    if (k < K) {
+        const float *src = buf + PITCH * r + k;
+        dst += STRIDE * k + r;
+        mask >>= k;
 #pragma unroll
-    for (int i = 0; i < R; ++i) {
-        const int e = lane + 32 * i, k = e / R, r = e - R * k;
-        if (mask >> k & 1u) dst[(ptrdiff_t)stride * k + r] = buf[33 * r + k];
+        for (int i = 0; i < 32; i += K)
+            if (mask >> i & 1u) dst[(ptrdiff_t)STRIDE * i] = src[i];
     }
 }
 

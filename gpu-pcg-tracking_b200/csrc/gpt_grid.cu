@@ -155,8 +155,9 @@ __global__ void __launch_bounds__(32 * FDG_WARPS)
 }
 
 // The same with one row per lane (gpt_fdlane.cuh), eight warps per SM (255 registers a thread, 26 KB of shared memory a
-// warp).  200,003 rows: 138 us against the half-warp form's 437, both cut by the issue of the tangent passes and their
-// latency (the rows' 685 bytes would take 21 us); two warps per CTA fill the last wave best (four 140, eight 154).
+// warp).  200,003 rows: 128 us against the half-warp form's 437, both cut by the issue of the tangent passes and their
+// latency (the rows' 685 bytes would take 21 us); two warps per CTA fill the last wave best (four 1%
+// more, eight 11%).
 constexpr int FDGL_WARPS = 2;
 
 __global__ void __launch_bounds__(32 * FDGL_WARPS, 8 / FDGL_WARPS)
@@ -179,18 +180,18 @@ __global__ void __launch_bounds__(32 * FDGL_WARPS, 8 / FDGL_WARPS)
     }
     JointTrig t;
     joint_trig(q, t);
-    fd_gradient_lane(t, qd, u, qdd, sm, lane, [&](int col, const float (&v)[NQ]) {
-        store_rows<NQ>(sm.out, v, df_out + NQ * NX * i0 + NQ * col, NQ * NX, mask, lane);
+    fd_gradient_lane(t, qd, u, qdd, sm, lane, [&](auto blk, int col, const float (&v)[NQ]) {
+        store_rows<NQ, NQ * NX>(sm.out, v, df_out + NQ * NX * i0 + CC * blk.block + NQ * col, mask, lane);
     });
-    store_rows<NQ>(sm.out, qdd, qdd_out + NQ * i0, NQ, mask, lane);
+    store_rows<NQ, NQ>(sm.out, qdd, qdd_out + NQ * i0, mask, lane);
 }
 
 cudaError_t launch_fd_grad(uint32_t n, const float *xu, uint32_t stride, float *qdd, float *df, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
-    // One row per lane from FDGL_MIN rows on: up to four warps per SM (18,944 rows) that form takes 21 us whatever the
-    // number of rows, the half-warp form 2.5 us per 1,000 rows beyond its own 4 (8,000 rows 23.7 against 21.2 us, 16,000
-    // rows 40.3 against 21.2)
+    // One row per lane from FDGL_MIN rows on: up to four warps per SM (18,944 rows) that form takes 19.5 us whatever the
+    // number of rows, the half-warp form 2.5 us per 1,000 rows beyond its own 4 (8,000 rows 23.6 against 19.4 us, 16,000
+    // rows 40.3 against 19.5)
     constexpr uint32_t FDGL_MIN = 8192;
     if (n >= FDGL_MIN) {
         constexpr int per = 32 * FDGL_WARPS;

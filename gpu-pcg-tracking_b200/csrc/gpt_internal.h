@@ -73,6 +73,8 @@ cudaError_t launch_pcg_part(const BatchView &bv, int max_n, int fmt, const void 
                             int num_sms, cudaStream_t s, bool warm = false);
 // its warps per instance for a batch of B instances (BatchView::part_warps carries it to part-batch views)
 int part_warps(int B, int max_n, int num_sms);
+// whether a batch's KKT formation (KKT_G_NONE) takes one knot per lane
+bool kkt_lane(int total_knots, int max_n);
 // lambda64 (optional) replaces lambda when given; Ginv64c (optional): the compact inverses of
 // launch_schur64 (GC64 doubles per knot), with Ginv64 holding only the blocks its flags name
 cudaError_t launch_dz(const BatchView &bv, const float *Ginv, const double *Ginv64, const double *Ginv64c,

@@ -20,6 +20,7 @@
 // written once per solve by gconst_kernel.
 #include "gpt_common.cuh"
 #include "gpt_dyn.cuh"
+#include "gpt_fdlane.cuh"
 #include "gpt_internal.h"
 
 namespace gpt {
@@ -338,11 +339,122 @@ __global__ void gconst_kernel(BatchView bv, float qd_cost, float r_cost, float *
     }
 }
 
+// KKT formation with one knot per lane (gpt_fdlane.cuh), for batches; nothing of G is written (KKT_G_NONE).  A warp takes 32
+// consecutive knots of the view; lanes past the view, an instance's last knot and knots of inactive instances compute on
+// whatever state they find and store nothing but the last knot's cost gradient, the terminal one.  512 x 128 knots: 70 us
+// against the half-warp form's 170 (C, g, c and the inputs are 105 MB, 16 us); bound by the issue of the tangent passes
+// at eight warps per SM (255 registers).
+constexpr int KKTL_WARPS = 2;
+
+__global__ void __launch_bounds__(32 * KKTL_WARPS, 8 / KKTL_WARPS)
+    kkt_lane_kernel(BatchView bv, ProblemParams P, const float *__restrict__ xu, const float *__restrict__ goal,
+                    const float *__restrict__ xs, float *__restrict__ Cm, float *__restrict__ g, float *__restrict__ c)
+{
+    extern __shared__ float4 kktl_dyn_smem[];
+    const int lane = threadIdx.x & 31;
+    FdLaneSmem &sm = reinterpret_cast<FdLaneSmem *>(kktl_dyn_smem)[threadIdx.x >> 5];
+    const int j0 = bv.j0 + 32 * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5), jend = bv.j0 + bv.total_knots;
+    const int j = min(j0 + lane, jend - 1), b = bv.inst(j), N = bv.N(b), k = j - bv.off(b);
+    const bool live = j0 + lane < jend && bv.active(b), valid = live && k < N - 1;
+    if (!__syncthreads_or(valid)) return;  // converged instances only
+    const uint32_t mask = __ballot_sync(0xffffffffu, valid);
+    const float *x = xu + (size_t)NX * j;
+    float q[NQ], qd[NQ], u[NC], qdd[NQ];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+        q[i] = x[i];
+        qd[i] = x[NQ + i];
+        u[i] = valid ? x[NS + i] : 0.f;  // (an instance's last knot has no control)
+    }
+    JointTrig t;
+    joint_trig(q, t);
+    // ---- cost gradient (iiwa_eepos_plant.cuh:329-354), the terminal one by the last knot's lane
+    {
+        float ee[3], J[3 * NQ], gv[NS], gr[NC];
+        fk_lane<true>(t, ee, J);
+        const float *gl = goal + (size_t)6 * j;
+        auto grad = [&](float t0, float t1, float t2, float *out) {
+#pragma unroll
+            for (int i = 0; i < NQ; ++i) {
+                out[i] = P.q_ee * (J[3 * i] * (ee[0] - t0) + J[3 * i + 1] * (ee[1] - t1) + J[3 * i + 2] * (ee[2] - t2));
+                out[NQ + i] = P.qd_cost * qd[i];
+            }
+        };
+        grad(gl[0], gl[1], gl[2], gv);
+#pragma unroll
+        for (int i = 0; i < NC; ++i) gr[i] = P.r_cost * u[i];
+        const uint32_t states = __ballot_sync(0xffffffffu, live && (valid || !P.ref_terminal));
+        store_rows<NS, NX>(sm.out, gv, g + (size_t)NX * j0, states, lane);
+        store_rows<NC, NX>(sm.out, gr, g + (size_t)NX * j0 + NS, mask, lane);
+        if (P.ref_terminal && valid && k == N - 2) {
+            // the reference's overwritten terminal goal (see kkt_kernel)
+            float gt[NS];
+            grad(gv[0] * gv[0], gv[0] * gv[1], gv[0] * gv[2], gt);
+#pragma unroll
+            for (int i = 0; i < NS; ++i) g[(size_t)NX * (j + 1) + i] = gt[i];
+        }
+        if (valid && k == 0) {
+#pragma unroll
+            for (int i = 0; i < NS; ++i) c[(size_t)NS * j + i] = x[i] - xs[(size_t)NS * b + i];
+        }
+    }
+    // ---- C_k = {-A_k, -B_k} column by column (integrator.cuh:85-126, sign from schur.cuh:519-520)
+    const float dt = P.dt;
+    float *C0 = Cm + (size_t)C_STRIDE * j0;
+    fd_gradient_lane(t, qd, u, qdd, sm, lane, [&](auto blk, int col, const float (&df)[NQ]) {
+        float v[NS];
+#pragma unroll
+        for (int r = 0; r < NQ; ++r) {
+            const float one = r == col ? 1.f : 0.f;  // the entry's identity part
+            v[r] = P.integrator == 0 ? 0.f : dt * df[r] * dt;
+            v[NQ + r] = dt * df[r];
+            if (blk.block == 0) v[r] += one;
+            if (blk.block == 1) {
+                v[r] += dt * one;
+                v[NQ + r] += one;
+            }
+            v[r] = -v[r];
+            v[NQ + r] = -v[NQ + r];
+        }
+        store_rows<NS, C_STRIDE>(sm.out, v, C0 + SS * blk.block / 2 + NS * col, mask, lane);
+    });
+    // ---- defect c_{k+1} = x_{k+1} - f(x_k, u_k)  (integrator.cuh:25-83)
+    float cn[NS];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+        float nq, nqd;
+        if (P.integrator == 0) {
+            nq = q[i] + dt * qd[i];
+            nqd = qd[i] + dt * qdd[i];
+        } else {
+            nqd = qd[i] + dt * qdd[i];
+            nq = q[i] + dt * nqd;
+        }
+        cn[i] = valid ? x[NX + i] - nq : 0.f;
+        cn[NQ + i] = valid ? x[NX + NQ + i] - nqd : 0.f;
+    }
+    store_rows<NS, NS>(sm.out, cn, c + (size_t)NS * (j0 + 1), mask, lane);
+}
+
+// One knot per lane from 9216 knots on: up to four warps per SM (18,944 knots) a launch of that form takes 29 to 36 us, the
+// half-warp form 25.8 at 6,192 knots, 30 at 8,256, 39.4 at 12,384 and 49.2 at 16,512; at 65,536 the two take 70 and
+// 170 us.  The two differ by FP32 rounding, which a solve amplifies with its horizon (a step's multipliers at 128 knots by
+// 1e-6 of their size, at 511 knots by 3e-5), so longer horizons stay with the half-warp form, whose results they have.
+bool kkt_lane(int total_knots, int max_n) { return total_knots >= 9216 && max_n <= 128; }
+
 cudaError_t launch_kkt(const BatchView &bv, const ProblemParams &P, const float *xu, const float *goal,
                        const float *xs, float *G, float *C, float *g, float *c, int num_sms, cudaStream_t s,
                        int ctas_per_sm, int g_mode)
 {
     if (bv.total_knots <= 0) return cudaSuccess;
+    if (g_mode == KKT_G_NONE && bv.kkt_lane) {
+        const size_t smem = sizeof(FdLaneSmem) * KKTL_WARPS;
+        const cudaError_t e = ensure_func_attrs((const void *)kkt_lane_kernel, smem);
+        if (e != cudaSuccess) return e;
+        const int per = 32 * KKTL_WARPS;
+        kkt_lane_kernel<<<(bv.total_knots + per - 1) / per, per, smem, s>>>(bv, P, xu, goal, xs, C, g, c);
+        return cudaGetLastError();
+    }
     int warps = (bv.total_knots + 1) / 2;  // two knots per warp
     int blocks = (warps + KKT_WARPS - 1) / KKT_WARPS;
     const int cap = num_sms * ctas_per_sm;
