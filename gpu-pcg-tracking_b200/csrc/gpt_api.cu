@@ -721,7 +721,7 @@ static gpt_status setup_batch(gpt_handle *h, uint32_t B, const uint32_t *Ns, con
     bv.knot_off = h->knot_off;
     bv.knot_inst = h->knot_inst;
     bv.st = h->st;
-    bv.part_warps = part_warps((int)B, maxN, h->num_sms);
+    bv.part_variant = part_variant((int)B, maxN, h->num_sms);
     bv.kkt_lane = kkt_lane(total, maxN);
     maxN_out = maxN;
     minN_out = minN;

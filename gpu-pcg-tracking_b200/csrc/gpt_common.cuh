@@ -57,9 +57,8 @@ struct BatchView {
     // A view of a contiguous sub-range of a batch: instances b0 .. b0+B-1, owning knots
     // j0 .. j0+total_knots-1.  Instance and knot indices stay those of the whole batch.
     int j0 = 0, b0 = 0;
-    // the partitioned PCG's warps per instance, fixed by the whole batch so that its parts give the same bits
-    // (0: by this view)
-    int part_warps = 0;
+    // the partitioned PCG's variant, fixed by the whole batch so that its parts give the same bits (0: by this view)
+    int part_variant = 0;
     // KKT formation with one knot per lane (a choice for the whole batch too)
     bool kkt_lane = false;
 

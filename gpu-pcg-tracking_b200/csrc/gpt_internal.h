@@ -71,8 +71,10 @@ cudaError_t launch_pcg_part(const BatchView &bv, int max_n, int fmt, const void 
                             const double *gamma64, float *lambda, double *lambda64, double *ws, int max_iter,
                             float tol, int exit_mode, uint32_t *out_iters, uint32_t *pcg_log, int log_stride,
                             int num_sms, cudaStream_t s, bool warm = false);
-// its warps per instance for a batch of B instances (BatchView::part_warps carries it to part-batch views)
-int part_warps(int B, int max_n, int num_sms);
+// its variants, by the parts of an instance (8X2: on two CTAs), and the one for a batch of B instances
+// (BatchView::part_variant carries it to part-batch views)
+enum { PART_2 = 2, PART_4 = 4, PART_8 = 8, PART_8X2 = 9, PART_16 = 16, PART_32 = 32 };
+int part_variant(int B, int max_n, int num_sms);
 // whether a batch's KKT formation (KKT_G_NONE) takes one knot per lane
 bool kkt_lane(int total_knots, int max_n);
 // lambda64 (optional) replaces lambda when given; Ginv64c (optional): the compact inverses of

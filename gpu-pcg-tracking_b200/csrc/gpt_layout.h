@@ -38,8 +38,16 @@ GPT_HD inline PartLayout<NW> part_layout(int n, int edge)
         len[0] = nint / 2;
         len[1] = nint - len[0];
     } else {
-        const int y = (10 * nint) / (2 * edge + 10 * (P - 2));
-        const int rest = nint - (P - 2) * y;
+        // the balanced length of a middle part rounded down, or up where that makes the longest walk shorter (a step of
+        // a middle part takes edge tenths of an edge part's; sixteen parts of 128 knots: edges of 14 and 15 knots
+        // beside middles of 6, or of 7 and 8 beside 7)
+        int y = (10 * nint) / (2 * edge + 10 * (P - 2));
+        int rest = nint - (P - 2) * y;
+        const int up = rest - (P - 2), walk = edge * y > 5 * (rest + 1) ? edge * y : 5 * (rest + 1);
+        if (up >= 0 && edge * (y + 1) < walk && 5 * (up + 1) < walk) {
+            ++y;
+            rest = up;
+        }
         len[0] = rest / 2;
         for (int p = 1; p < P - 1; ++p) len[p] = y;
         len[P - 1] = rest - len[0];

@@ -1,5 +1,5 @@
-// gpt_part.cu -- the partitioned PCG (pcg_cluster_size PCG_WARP_QUAD): one CTA per instance whose
-// warps factor parts of the horizon.
+// gpt_part.cu -- the partitioned PCG (pcg_cluster_size PCG_WARP_QUAD): one CTA or one cluster of CTAs per
+// instance, whose warps factor parts of the horizon.
 //
 // Solves S lambda = gamma by conjugate gradients with the exact inverse of S as the preconditioner
 // (z = S^{-1} r up to rounding), so the iteration stops after one step; it starts from lambda = 0
@@ -7,8 +7,8 @@
 // E_k = M_{k,k-1} = -L_k (L_k the left block of row k of S), the horizon is cut by P - 1 separator
 // knots s_1 < ... < s_{P-1} into P parts.  Part 0 is eliminated top-down toward s_1 and part P-1
 // bottom-up toward s_{P-1}; a middle part top-down from its left to its right separator, which couples
-// the two.  The separators' block-tridiagonal system is eliminated by one warp, then every part is
-// solved backward.  This is the block L D L^T of M with the parts' knots ordered before the
+// the two.  The separators' block-tridiagonal system is eliminated by two warps from both ends, then every
+// part is solved backward.  This is the block L D L^T of M with the parts' knots ordered before the
 // separators.
 //
 // One elimination step (part_step) is the symmetric elimination of the 14 unknowns of one knot from
@@ -36,11 +36,15 @@
 // Storage per knot: QW_STRIDE doubles of the FP64 workspace: L^{-1} (QINV), F_k row-major (SS), S x, and,
 // only when the iteration goes on, the CG vectors.  S is read from global memory in rows staged by
 // cp.async.
+#include <cooperative_groups.h>
+
 #include <type_traits>
 
 #include "gpt_common.cuh"
 #include "gpt_internal.h"
 #include "gpt_layout.h"
+
+namespace cg = cooperative_groups;
 
 namespace gpt {
 
@@ -64,20 +68,22 @@ constexpr int QROWS_D = 2 * 2 * 37;        // pivot rows: 2 sets of 2 rows (D, E
 constexpr int QBUF = QROWS_D + 2 * NS;     // pivot rows; B^{-1} by rows
 constexpr int RR_PERIOD = 32;              // CG iterations between true-residual replacements
 
-// A kernel variant: NW warps per instance, SL staging slots per warp, MINB CTAs per SM, EDGE the length of an
-// edge part in tenths of a middle part's
-template <int NW_, int SL_, int MINB_, int EDGE_>
+// A kernel variant: a cluster of CL CTAs of WC warps per instance (NW = CL WC parts, in order over the CTAs), SL staging
+// slots per warp, MINB CTAs per SM, EDGE the length of an edge part in tenths of a middle part's
+template <int CL_, int WC_, int SL_, int MINB_, int EDGE_>
 struct PartCfg {
-    static_assert(NW_ >= 2 && SL_ >= 3, "two parts, three slots at least");
-    static constexpr int NW = NW_, SL = SL_, MINB = MINB_, EDGE = EDGE_;
+    static_assert(WC_ >= 2 && SL_ >= 3, "two warps, three slots at least");
+    static constexpr int CL = CL_, WC = WC_, NW = CL * WC, SL = SL_, MINB = MINB_, EDGE = EDGE_;
     static constexpr int REGION = SL * QSLOT_D;
     static constexpr int SB = REGION / QBACK_D;  // slots of the backward sweep
-    // the middle parts' W; after the walks the separators' L^{-1} and right-hand-side terms
-    static constexpr int MID =
-        (NW - 2) * QW_D > (NW - 1) * (QINV + NS) ? (NW - 2) * QW_D : (NW - 1) * (QINV + NS);
+    // the middle parts' W; after the walks the separators' L^{-1}, the bottom half's update of the middle one and the
+    // terms of S x that belong to a separator
+    static constexpr int MIDS = CL == 1 ? NW - 2 : WC;
+    static constexpr int SEP_B = (NW - 1) * QINV, SEP_SX = SEP_B + (NW > 2 ? QSEP : 0);
+    static constexpr int MID = MIDS * QW_D > SEP_SX + WC * NS ? MIDS * QW_D : SEP_SX + WC * NS;
     static size_t smem_bytes(int n)
     {
-        return sizeof(double) * (size_t)(NS * n + NW * (REGION + QBUF) + MID + 2 * NW * 3);
+        return sizeof(double) * (size_t)(NS * n + WC * (REGION + QBUF) + MID + 2 * NW * 3 + 4);
     }
 };
 
@@ -328,15 +334,38 @@ struct PartRows {
 template <class CF>
 struct PartSmem {
     double *stg, *buf, *wmid, *red, *xv;
+    int *lay;
     __device__ __forceinline__ explicit PartSmem(double *base)
     {
         stg = base;                         // per warp: staged rows / steps; the separators' blocks
-        buf = stg + CF::NW * CF::REGION;    // per warp: pivot rows; the backward sweep's scratch
-        wmid = buf + CF::NW * QBUF;
+        buf = stg + CF::WC * CF::REGION;    // per warp: pivot rows; the backward sweep's scratch
+        wmid = buf + CF::WC * QBUF;
         red = wmid + CF::MID;               // 2 sets x NW warps x 3
-        xv = red + 2 * CF::NW * 3;          // 14 n: y, then z, then x
+        lay = reinterpret_cast<int *>(red + 2 * CF::NW * 3);  // parts, first separator, spacing, this CTA's knots
+        xv = red + 2 * CF::NW * 3 + 4;      // 14 n: y, then z, then x (of the CTA's knots and all separators)
     }
 };
+
+// barrier over the instance's threads
+template <class CF>
+__device__ __forceinline__ void part_sync()
+{
+    if constexpr (CF::CL == 1) __syncthreads();
+    else cg::this_cluster().sync();
+}
+template <class CF>
+__device__ __forceinline__ int part_rank()
+{
+    if constexpr (CF::CL == 1) return 0;
+    else return (int)cg::this_cluster().block_rank();
+}
+// address p of this CTA's shared memory in CTA r of the cluster
+template <class CF>
+__device__ __forceinline__ double *part_peer(double *p, int r)
+{
+    if constexpr (CF::CL == 1) return p;
+    else return cg::this_cluster().map_shared_rank(p, r);
+}
 
 // The elimination of one part (knots pa .. pb; SPK: a middle part) by the calling warp: L^{-1} (and F) of
 // every knot into the workspace, z into xv, and into the warp's staging region, in the lane layout, its
@@ -407,7 +436,7 @@ __device__ __forceinline__ void walk_part(const typename std::conditional<FMT ==
                 for (int q = 0; q < 7; ++q) wf[28 * q] = f[q];
             }
             // row st is done with: its slot holds V
-            part_step_mid(a, e, f, b, acc, buf, ps.wmid + (warp - 1) * QW_D, s0, lane);
+            part_step_mid(a, e, f, b, acc, buf, ps.wmid + (CF::CL == 1 ? warp - 1 : warp) * QW_D, s0, lane);
             double d[7];
             ld_block(s1, k0 + st + 1, d);  // a middle part ends at a separator: the next row exists
 #pragma unroll
@@ -484,7 +513,7 @@ struct PartCtx {
     {
         int cta;
         asm volatile("mov.u32 %0, %%ctaid.x;" : "=r"(cta));
-        inst = A.bv.b0 + cta;
+        inst = A.bv.b0 + cta / CF::CL;
         n = A.bv.N(inst);
         kg0 = A.bv.off(inst);
     }
@@ -510,78 +539,129 @@ __device__ __forceinline__ void part_apply(const PartArgs &A)
     extern __shared__ __align__(16) double part_dyn_smem[];
     const PartSmem<CF> ps(part_dyn_smem);
     const PartCtx<FMT, CF> cx(A);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, rank = part_rank<CF>(), part = rank * CF::WC + warp;
     const int c = lane >> 1, h = lane & 1, cl = c < NS ? c : NS - 1;
     const int n = cx.n;
-    int P, len0, step;  // parts; separators at len0 + j step
-    {
-        const PartLayout<NW> lay = part_layout<NW>(n, CF::EDGE);
-        P = lay.P;
-        len0 = lay.s[0];
-        step = NW > 2 ? lay.s[NW > 2 ? 1 : 0] - lay.s[0] : 0;
-    }
+    part_sync<CF>();
+    const int P = ps.lay[0], len0 = ps.lay[1], step = ps.lay[2];  // separators at len0 + j step
     auto sep_of = [&](int j) { return len0 + j * step; };
-    const bool mid = warp > 0 && warp < P - 1, top = warp < P - 1 || P == 1;
-    const int pa = warp == 0 ? 0 : sep_of(warp - 1) + 1, pb = warp >= P - 1 ? n - 1 : sep_of(warp) - 1;
+    const bool mid = part > 0 && part < P - 1, top = part < P - 1 || P == 1;
+    const int pa = part == 0 ? 0 : sep_of(part - 1) + 1, pb = part >= P - 1 ? n - 1 : sep_of(part) - 1;
     double *xv = ps.xv, *scw = ps.buf + warp * QBUF;
-    __syncthreads();
-    if (warp < P) {
+    if (part < P) {
         if (mid) walk_part<FMT, CF, true>(cx.rows(), cx.work(), pa, pb, true, true);
         else walk_part<FMT, CF, false>(cx.rows(), cx.work(), pa, pb, top, P > 1);
     }
-    __syncthreads();
-    // ---- the separators' system, by warp 0
-    if (warp == 0 && P >= 2) {
+    part_sync<CF>();
+    // ---- the separators' system, by two warps of CTA 0: from both ends toward the middle separator sm and back (one
+    // warp's chain over all of them is twice as long: seven took 20 k cycles)
+    if (rank == 0 && warp < 2 && P >= 2) {
+        const int sm = (P - 1) >> 1;  // of P - 1 separators
+        const bool down = warp == 0;
+        const int dj = down ? 1 : -1, js = down ? 0 : P - 2, cnt = down ? sm : P - 2 - sm;
         double a[7], e[7], b[7];
         auto rinv = [&](int j) { return ps.wmid + j * QINV; };
-        auto sep = [&](int j, int q) -> double {
-            const double *l = ps.stg + j * CF::REGION;
-            const double *r = ps.stg + (j + 1) * CF::REGION + (j + 1 < P - 1 ? QSEP : 0);
-            return l[32 * q + lane] + r[32 * q + lane];
+        auto region = [&](int p) { return part_peer<CF>(ps.stg + (p % CF::WC) * CF::REGION, p / CF::WC); };
+        auto sep = [&](int j, double (&v)[7]) {
+            const double *l = region(j) + lane, *r = region(j + 1) + (j + 1 < P - 1 ? QSEP : 0) + lane;
+#pragma unroll
+            for (int q = 0; q < 7; ++q) v[q] = l[32 * q] + r[32 * q];
         };
-        // M_{s_{j+1}, s_j}, or an initialised block when there is none
-        auto cpl = [&](int j) { return ps.stg + (j + 1) * CF::REGION + (j + 1 < P - 1 ? 2 * QSEP : 0); };
+        // row i, column k of M_{s_{j+1}, s_j} at 32 (i >> 1) + 2 k + (i & 1)
+        auto cpl = [&](int j) { return region(j + 1) + 2 * QSEP; };
+        // E^T of separator j toward the middle: M_{s_{j+1}, s_j}^T, or M_{s_j, s_{j-1}}
+        auto coup = [&](int j, double (&v)[7]) {
+            const double *E = down ? cpl(j) + 32 * (cl >> 1) + (cl & 1) + 2 * h : cpl(j - 1) + 2 * cl + h;
 #pragma unroll
-        for (int q = 0; q < 7; ++q) b[q] = sep(0, q);
-        for (int j = 0; j < P - 1; ++j) {
-            const double *Eh = cpl(j) + 32 * (cl >> 1) + (cl & 1) + 2 * h;
-            const bool more = j + 1 < P - 1;
-            const int jn = more ? j + 1 : j;
-#pragma unroll
-            for (int q = 0; q < 7; ++q) {
-                const double ev = Eh[4 * q], bv = sep(jn, q);
-                a[q] = b[q];
-                e[q] = c < NS ? (more ? ev : 0.0) : b[q];
-                b[q] = more ? bv : 0.0;
-            }
-            part_step(a, e, b, scw, lane);
+            for (int q = 0; q < 7; ++q) v[q] = E[(down ? 4 : 32) * q];
+        };
+        auto keep = [&](int j) {
 #pragma unroll
             for (int q = 0; q < 7; ++q) {
                 if (c <= 2 * q + h && c < NS) rinv(j)[2 * q * (q + 1) + lane] = a[q];
                 if (c == NS) xv[NS * sep_of(j) + 2 * q + h] = e[q];
             }
-        }
-        __syncwarp();
-        for (int j = P - 2; j >= 0; --j) {
-            PartBack pk;
-            pk.load(rinv(j), lane);
-            double t = 0.0;
-            if (j + 1 < P - 1) {
-                const double *Eh = cpl(j) + 2 * cl + h, *xn = xv + NS * sep_of(j + 1) + h;
+        };
+        if (cnt > 0) {
+            double en[7], bn[7];
+            sep(js, b);
+            coup(js, en);
+            for (int i = 0; i < cnt; ++i) {
+                const int j = js + dj * i;
+                if (down || i + 1 < cnt) {
+                    sep(j + dj, bn);
+                } else {
 #pragma unroll
-                for (int q = 0; q < 7; ++q) t = fma(-Eh[32 * q], xn[2 * q], t);
-                t += __shfl_xor_sync(0xffffffffu, t, 1);
+                    for (int q = 0; q < 7; ++q) bn[q] = 0.0;  // the middle one: its block is warp 0's
+                }
+#pragma unroll
+                for (int q = 0; q < 7; ++q) {
+                    a[q] = b[q];
+                    e[q] = c < NS ? en[q] : b[q];
+                    b[q] = bn[q];
+                }
+                if (i + 1 < cnt) coup(j + dj, en);
+                part_step(a, e, b, scw, lane);
+                keep(j);
             }
+        } else if (down) {
+            sep(sm, b);
+        }
+        double *upd = ps.wmid + CF::SEP_B + lane;
+        PartBack pk;
+        if constexpr (NW > 2) {
+            if (!down) {
+#pragma unroll
+                for (int q = 0; q < 7; ++q) upd[32 * q] = cnt > 0 ? b[q] : 0.0;
+            }
+            asm volatile("bar.sync 1, 64;" ::: "memory");
+        }
+        if (down) {
+            double zero[7];
+#pragma unroll
+            for (int q = 0; q < 7; ++q) {
+                if constexpr (NW > 2) b[q] += upd[32 * q];
+                a[q] = b[q];
+                e[q] = c < NS ? 0.0 : b[q];
+                zero[q] = 0.0;
+            }
+            part_step(a, e, zero, scw, lane);
+            keep(sm);
+            __syncwarp();
+            pk.load(rinv(sm), lane);
+            pk.step(0.0, xv + NS * sep_of(sm), scw, lane);
+        }
+        if constexpr (NW > 2) asm volatile("bar.sync 1, 64;" ::: "memory");
+        for (int i = cnt - 1; i >= 0; --i) {  // x_j from its neighbour toward the middle
+            const int j = js + dj * i;
+            const double *E = down ? cpl(j) + 2 * cl + h : cpl(j - 1) + 32 * (cl >> 1) + (cl & 1) + 2 * h;
+            const double *xh = xv + NS * sep_of(j + dj) + h;
+            double t = 0.0;  // -E^T x
+#pragma unroll
+            for (int q = 0; q < 7; ++q) t = fma(-E[(down ? 32 : 4) * q], xh[2 * q], t);
+            t += __shfl_xor_sync(0xffffffffu, t, 1);
+            pk.load(rinv(j), lane);
             pk.step(t, xv + NS * sep_of(j), scw, lane);
         }
+        if constexpr (CF::CL > 1) {  // to the other CTAs
+            const int j0 = down ? 0 : sm + 1, nj = down ? sm + 1 : cnt;
+            __syncwarp();
+            for (int i = lane; i < NS * nj; i += 32) {
+                const int e0 = NS * sep_of(j0 + i / NS) + i % NS;
+                const double x = xv[e0];
+#pragma unroll
+                for (int r = 1; r < CF::CL; ++r) part_peer<CF>(xv, r)[e0] = x;
+            }
+        }
     }
-    __syncthreads();
+    part_sync<CF>();
     // ---- backward through every part, and S x with it: a staged step is L^{-1} of the knot it solves and a row
     // of S.  Top-down parts go through the rows r = right separator .. pa: t = L_r^T x_r, then x_{r-1}, then row r
     // of S x; the last part through the rows r = pa .. pb: t = L_r x_{r-1}, then x_r, then row r - 1 of S x.
     // L_pa^T x_pa belongs to the left separator's row (sacc).
-    double *sacc = ps.wmid + (NW - 1) * QINV;
-    if (warp < P) {
+    double *sacc = ps.wmid + CF::SEP_SX;
+    double *sleft = part > 0 ? part_peer<CF>(sacc, (part - 1) / CF::WC) + NS * ((part - 1) % CF::WC) : sacc;
+    if (part < P) {
         double *stg = ps.stg + warp * CF::REGION;
         const ST *Sb = cx.rows();
         double *wsb = cx.work();
@@ -656,8 +736,8 @@ __device__ __forceinline__ void part_apply(const PartArgs &A)
                         if (k > pa) ld_f(k - 1);
                     }
                     pk.step(t + tf, xv + NS * k, scw, lane);
-                } else if (warp > 0 && wr) {
-                    sacc[NS * (warp - 1) + c] = t;
+                } else if (part > 0 && wr) {
+                    sleft[c] = t;
                 }
                 if (r > 0) {
                     ld_x(k);
@@ -674,7 +754,7 @@ __device__ __forceinline__ void part_apply(const PartArgs &A)
                 ld_x(r);
                 const double u = pair(dot(M + lc, 2, xr)), v = pair(dot_diag(M, xr));
                 if (wr) {
-                    if (i == 0) sacc[NS * (warp - 1) + c] = u;
+                    if (i == 0) sleft[c] = u;
                     else wsb[(ptrdiff_t)(r - 1) * QW_STRIDE + QW_SX + c] = carry + u;
                 }
                 carry = t + v;
@@ -683,27 +763,27 @@ __device__ __forceinline__ void part_apply(const PartArgs &A)
         cp_async_wait<0>();
         if (!top && wr) {
             if (count > 0) wsb[(ptrdiff_t)pb * QW_STRIDE + QW_SX + c] = carry;
-            else sacc[NS * (warp - 1) + c] = 0.0;
+            else sleft[c] = 0.0;
         }
     }
-    __syncthreads();
-    if (warp < P - 1 && lane < NS) cx.work()[(ptrdiff_t)sep_of(warp) * QW_STRIDE + QW_SX + lane] += sacc[NS * warp + lane];
+    part_sync<CF>();
+    if (part < P - 1 && lane < NS) cx.work()[(ptrdiff_t)sep_of(part) * QW_STRIDE + QW_SX + lane] += sacc[NS * warp + lane];
     __syncthreads();
 }
 
-// sums of v[0 .. CNT-1] over the CTA, in a fixed order (set: alternate between calls)
+// sums of v[0 .. CNT-1] over the instance's threads, in a fixed order (set: alternate between calls)
 template <class CF, int CNT>
 __device__ __forceinline__ void part_sum(double (&v)[CNT], int set)
 {
     extern __shared__ __align__(16) double part_dyn_smem[];
     double *red = PartSmem<CF>(part_dyn_smem).red + set * CF::NW * 3;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, part = part_rank<CF>() * CF::WC + (threadIdx.x >> 5);
 #pragma unroll
     for (int q = 0; q < CNT; ++q) {
         const double s = warp_sum(v[q]);
-        if (lane == 0) red[3 * warp + q] = s;
+        if (lane < CF::CL) part_peer<CF>(red, lane)[3 * part + q] = s;
     }
-    __syncthreads();
+    part_sync<CF>();
 #pragma unroll
     for (int q = 0; q < CNT; ++q) {
         double s = 0.0;
@@ -711,6 +791,19 @@ __device__ __forceinline__ void part_sum(double (&v)[CNT], int set)
         v[q] = s;
     }
 }
+
+// the vector entries of this CTA's knots, from this thread's first one on (every 32 WC-th is its own)
+template <class CF>
+struct PartRange {
+    int first, end;
+    __device__ __forceinline__ PartRange()
+    {
+        extern __shared__ __align__(16) double part_dyn_smem[];
+        const int *lay = PartSmem<CF>(part_dyn_smem).lay;
+        first = NS * lay[3] + threadIdx.x;
+        end = NS * lay[4];
+    }
+};
 
 // r = gamma - S lambda (the workspace's lambda) into the workspace and r . r; a rare path
 template <int FMT, class CF>
@@ -720,8 +813,9 @@ __device__ __noinline__ double part_true_residual(const PartArgs &A, int set)
     const typename PartRows<FMT>::ST *Sb = cx.rows();
     constexpr ptrdiff_t ks = PartCtx<FMT, CF>::ks;
     double s[1] = {0.0};
-    __syncthreads();
-    for (int e = threadIdx.x; e < NS * cx.n; e += 32 * CF::NW) {
+    part_sync<CF>();
+    const PartRange<CF> rg;
+    for (int e = rg.first; e < rg.end; e += 32 * CF::WC) {
         const int k = e / NS, i = e % NS;
         const typename PartRows<FMT>::ST *row = Sb + ks * k;
         double a = 0.0;
@@ -739,26 +833,44 @@ __device__ __noinline__ double part_true_residual(const PartArgs &A, int set)
 }
 
 template <int FMT, class CF>
-__global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const __grid_constant__ PartArgs A)
+__global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const __grid_constant__ PartArgs A)
 {
     static_assert(FMT == 1 || FMT == 2, "packed rows only");
-    constexpr int NT = 32 * CF::NW;
+    constexpr int NT = 32 * CF::WC;
     extern __shared__ __align__(16) double part_dyn_smem[];
     double *xv = PartSmem<CF>(part_dyn_smem).xv;
     const int tid = threadIdx.x;
     {
         const PartCtx<FMT, CF> cx(A);
-        if (!A.bv.active(cx.inst)) return;
-        for (int e = tid; e < NS * cx.n; e += NT) xv[e] = cx.gam(e);
+        if (!A.bv.active(cx.inst)) return;  // (the whole cluster)
+        int lo = 0, hi = cx.n;
+        const PartLayout<CF::NW> L = part_layout<CF::NW>(cx.n, CF::EDGE);
+        const int sep_step = CF::NW > 2 ? L.s[CF::NW > 2 ? 1 : 0] - L.s[0] : 0;
+        if constexpr (CF::CL > 1) {  // the CTA's parts and their right separators
+            const int f = part_rank<CF>() * CF::WC, l = f + CF::WC - 1;
+            lo = f == 0 ? 0 : (f < L.P ? L.s[0] + (f - 1) * sep_step + 1 : cx.n);
+            hi = l >= L.P - 1 ? cx.n : L.s[0] + l * sep_step + 1;
+        }
+        if (tid == 0) {
+            int *lay = PartSmem<CF>(part_dyn_smem).lay;
+            lay[0] = L.P;
+            lay[1] = L.s[0];
+            lay[2] = sep_step;
+            lay[3] = lo;
+            lay[4] = hi;
+        }
+        for (int e = NS * lo + tid; e < NS * hi; e += NT) xv[e] = cx.gam(e);
     }
     int it = 0, set = 0;
     bool conv = false, bad = false, in_xv = false;
     bool has_res = false;  // r and lambda are in the workspace (before: r = gamma, lambda = 0)
     double eta = 0.0, gg = 0.0, alpha = 0.0;
     if (A.warm) {
+        part_sync<CF>();
         const PartCtx<FMT, CF> cx(A);
+        const PartRange<CF> rg;
         double g2[2] = {0.0, 0.0};  // gamma . gamma; entries of lambda that are not 0
-        for (int e = tid; e < NS * cx.n; e += NT) {
+        for (int e = rg.first; e < rg.end; e += NT) {
             const double lam = (double)A.lambda[NS * cx.kg0 + e];
             cx.vec(QW_LAM, e) = lam;
             g2[0] = fma(xv[e], xv[e], g2[0]);
@@ -768,7 +880,7 @@ __global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const _
         if (g2[1] > 0.0) {
             gg = g2[0];
             part_true_residual<FMT, CF>(A, set ^ 1);
-            for (int e = tid; e < NS * cx.n; e += NT) xv[e] = cx.vec(QW_RES, e);
+            for (int e = rg.first; e < rg.end; e += NT) xv[e] = cx.vec(QW_RES, e);
             has_res = true;
         } else {
             set ^= 1;
@@ -780,14 +892,30 @@ __global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const _
     for (;;) {
         part_apply<FMT, CF>(A);
         const PartCtx<FMT, CF> cx(A);
-        const int nv = NS * cx.n;
+        const PartRange<CF> rg;
         double dd[3] = {0.0, 0.0, 0.0};  // r . z, r . r with z = -x; x . S x
-        for (int e = tid; e < nv; e += NT) {
-            const double r = has_res ? cx.vec(QW_RES, e) : cx.gam(e), x = xv[e];
+        // the thread's first KEEP entries of r and S x stay in registers for the new residual's norm
+        constexpr int KEEP = 8;
+        double rk[KEEP], sk[KEEP];
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i) {
+            const int e = rg.first + NT * i;
+            rk[i] = sk[i] = 0.0;
+            if (e < rg.end) {
+                rk[i] = has_res ? cx.vec(QW_RES, e) : cx.gam(e);
+                sk[i] = cx.vec(QW_SX, e);
+            }
+        }
+        auto dots = [&](double r, double x, double sx) {
             dd[0] = fma(-x, r, dd[0]);
             dd[1] = fma(r, r, dd[1]);
-            dd[2] = fma(x, cx.vec(QW_SX, e), dd[2]);
-        }
+            dd[2] = fma(x, sx, dd[2]);
+        };
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i)
+            if (rg.first + NT * i < rg.end) dots(rk[i], xv[rg.first + NT * i], sk[i]);
+        for (int e = rg.first + NT * KEEP; e < rg.end; e += NT)
+            dots(has_res ? cx.vec(QW_RES, e) : cx.gam(e), xv[e], cx.vec(QW_SX, e));
         part_sum<CF, 3>(dd, set);
         set ^= 1;
         if (it == 0) {
@@ -808,12 +936,15 @@ __global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const _
         if (it > 0) {        // p = z + beta p, S p = S z + beta S p
             const double beta = dd[0] / eta;
             double d1[1] = {0.0};
-            for (int e = tid; e < nv; e += NT) {
+            for (int e = rg.first; e < rg.end; e += NT) {
                 const double p = fma(beta, cx.vec(QW_P, e), -xv[e]), v = fma(beta, cx.vec(QW_V, e), -cx.vec(QW_SX, e));
                 xv[e] = -p;
                 cx.vec(QW_SX, e) = -v;
                 d1[0] = fma(p, v, d1[0]);
             }
+#pragma unroll
+            for (int i = 0; i < KEEP; ++i)
+                if (rg.first + NT * i < rg.end) sk[i] = cx.vec(QW_SX, rg.first + NT * i);
             part_sum<CF, 1>(d1, set);
             set ^= 1;
             psp = d1[0];
@@ -825,7 +956,12 @@ __global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const _
             break;
         }
         double r2[1] = {0.0};
-        for (int e = tid; e < nv; e += NT) {
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i) {
+            const double rn = fma(alpha, sk[i], rk[i]);
+            r2[0] = fma(rn, rn, r2[0]);
+        }
+        for (int e = rg.first + NT * KEEP; e < rg.end; e += NT) {
             const double rn = fma(alpha, cx.vec(QW_SX, e), has_res ? cx.vec(QW_RES, e) : cx.gam(e));
             r2[0] = fma(rn, rn, r2[0]);
         }
@@ -836,7 +972,7 @@ __global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const _
             conv = in_xv = true;  // lambda = alpha p
             break;
         }
-        for (int e = tid; e < nv; e += NT) {
+        for (int e = rg.first; e < rg.end; e += NT) {
             cx.vec(QW_RES, e) = fma(alpha, cx.vec(QW_SX, e), has_res ? cx.vec(QW_RES, e) : cx.gam(e));
             cx.vec(QW_LAM, e) = fma(-alpha, xv[e], has_res ? cx.vec(QW_LAM, e) : 0.0);
             cx.vec(QW_P, e) = -xv[e];
@@ -863,15 +999,16 @@ __global__ void __launch_bounds__(32 * CF::NW, CF::MINB) pcg_part_kernel(const _
                 break;
             }
         }
-        for (int e = tid; e < nv; e += NT) xv[e] = cx.vec(QW_RES, e);
+        for (int e = rg.first; e < rg.end; e += NT) xv[e] = cx.vec(QW_RES, e);
     }
     const PartCtx<FMT, CF> cx(A);
-    for (int e = tid; e < NS * cx.n; e += NT) {
+    const PartRange<CF> rg;
+    for (int e = rg.first; e < rg.end; e += NT) {
         const double lam = in_xv ? -alpha * xv[e] : (has_res ? cx.vec(QW_LAM, e) : 0.0);
         A.lambda[NS * cx.kg0 + e] = (float)lam;
         if (A.lambda64) A.lambda64[NS * cx.kg0 + e] = lam;
     }
-    if (tid == 0) {
+    if (tid == 0 && part_rank<CF>() == 0) {
         const int inst = cx.inst;
         const uint32_t maxit = conv ? 0u : 1u;
         if (A.out_iters) {
@@ -898,25 +1035,48 @@ static cudaError_t launch_part_t(const PartArgs &A, int max_n, cudaStream_t s)
     const size_t smem = CF::smem_bytes(max_n);
     const cudaError_t e = ensure_func_attrs((const void *)kern, smem);
     if (e != cudaSuccess) return e;
-    kern<<<A.bv.B, 32 * CF::NW, smem, s>>>(A);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = A.bv.B * CF::CL;
+    cfg.blockDim = 32 * CF::WC;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = CF::CL;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = CF::CL > 1 ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kern, A);
 }
 
 // The variants: every warp of them has 255 registers (at 128, which four 4-warp CTAs per SM need, the
 // elimination's loads serialise: 1.8 k -> 2.8 k cycles per edge step of a lone warp), so eight warps share an SM.
 // Staging slots: the few-instance variants prefetch deeper, their sweeps being bound by the latency of L2.
-using Part8 = PartCfg<8, 6, 1, 15>;
-using Part4 = PartCfg<4, 4, 2, 15>;
-using Part2 = PartCfg<2, 3, 4, 13>;
+using Part32 = PartCfg<8, 4, 6, 1, 15>;
+using Part16 = PartCfg<4, 4, 6, 1, 15>;
+using Part8x2 = PartCfg<2, 4, 6, 1, 15>;
+using Part8 = PartCfg<1, 8, 6, 1, 15>;
+using Part4 = PartCfg<1, 4, 4, 2, 15>;
+using Part2 = PartCfg<1, 2, 3, 4, 13>;
 
-// Warps per instance.  More parts shorten an instance's chain but add the middle parts' work (about 1.6 of
-// an edge part's per knot), and one, two or four CTAs of 8, 4 or 2 warps share an SM.  Measured, us per
-// launch (8 / 4 / 2 warps): n = 128, 1 instance 79 / 97 / 132, 148 instances 85 / 93 / 133; n = 64, 200 instances
-// 93 / 67 / 74, 400 instances 142 / 127 / 96; n = 32, 1 instance 35 / 34 / 42.
-int part_warps(int B, int max_n, int num_sms)
+// The variant of a batch.  More parts shorten an instance's chain but add the middle parts' work (about 1.6 of an edge
+// part's per knot) and a separator each to the two-sided chain (3.3 k cycles for two of them); a cluster spreads the parts
+// over SMs that would be idle, one warp per scheduler (2.4 k cycles per edge step against 3.3 k at two), and costs about
+// 1.3 k cycles per cluster barrier.  Measured, us per launch (1 CTA of 4 / 1 of 8 / 2 x 4 / 4 x 4 / 8 x 4 warps), one instance:
+// n = 16 20 / 20 / 29 / 24 / 25, n = 32 29 / 27 / 29 / 31 / 33, n = 48 40 / 37 / 35 / 36 / 41, n = 64 47 / 43 / 39 / 37 / 46,
+// n = 128 85 / 72 / 60 / 47 / 52, n = 200 127 / 105 / 85 / 60 / 61, n = 300 185 / 149 / 117 / 76 / 72, n = 511 308 / 244 / 189
+// / 113 / 85.  Clusters of 8 fit 14 or 15 times at once, of 4 33 times and of 2 74 times (n = 511, 16 instances: 166 us with
+// 8 x 4, 114 with 4 x 4; n = 128, 35 instances: 62 with 4 x 4, 61 with 2 x 4; n = 64, 74 instances: 40 with 2 x 4, 46 with 8).
+// Above one instance per SM 4 and 2 warps (us, 8 / 4 / 2 warps): n = 64, 200 instances 93 / 67 / 74, 400 instances
+// 142 / 127 / 96.
+int part_variant(int B, int max_n, int num_sms)
 {
-    if (B <= num_sms) return max_n >= 64 ? 8 : 4;
-    return B <= 2 * num_sms ? 4 : 2;
+    if (B > num_sms) return B <= 2 * num_sms ? PART_4 : PART_2;
+    if (max_n < 24) return PART_4;
+    if (max_n < 48) return PART_8;
+    if (max_n >= 256 && 12 * B <= num_sms) return PART_32;
+    if (9 * B <= 2 * num_sms) return PART_16;
+    return 2 * B <= num_sms ? PART_8X2 : PART_8;
 }
 
 template <class CF>
@@ -932,9 +1092,12 @@ cudaError_t launch_pcg_part(const BatchView &bv, int max_n, int fmt, const void 
 {
     const PartArgs A{bv,       S,         gamma,      gamma64, lambda,    lambda64, ws,
                      max_iter, exit_mode, log_stride, warm ? 1 : 0, tol, out_iters, pcg_log};
-    switch (bv.part_warps ? bv.part_warps : part_warps(bv.B, max_n, num_sms)) {
-    case 8: return launch_part_f<Part8>(A, max_n, fmt, s);
-    case 4: return launch_part_f<Part4>(A, max_n, fmt, s);
+    switch (bv.part_variant ? bv.part_variant : part_variant(bv.B, max_n, num_sms)) {
+    case PART_32: return launch_part_f<Part32>(A, max_n, fmt, s);
+    case PART_16: return launch_part_f<Part16>(A, max_n, fmt, s);
+    case PART_8X2: return launch_part_f<Part8x2>(A, max_n, fmt, s);
+    case PART_8: return launch_part_f<Part8>(A, max_n, fmt, s);
+    case PART_4: return launch_part_f<Part4>(A, max_n, fmt, s);
     default: return launch_part_f<Part2>(A, max_n, fmt, s);
     }
 }

@@ -1,4 +1,4 @@
-"""The partitioned PCG's variants (2, 4 and 8 warps per instance, chosen by the batch size and the longest
+"""The partitioned PCG's variants (2 to 32 parts per instance on 1 to 8 CTAs, chosen by the batch size and the longest
 horizon) at the edges of their ranges, and their part layouts.
 
 Tolerance: the multipliers are the FP64 solution of a system of condition up to about 2e7 (2.2e-16 x 2e7 x
@@ -36,7 +36,7 @@ template <int NW> int check(int edge)
 int main()
 {
     for (int edge = 13; edge <= 15; edge += 2)
-        if (int r = 10 * check<2>(edge) + 100 * check<4>(edge) + 1000 * check<8>(edge)) return r ? 1 : 0;
+        if (check<2>(edge) || check<4>(edge) || check<8>(edge) || check<16>(edge) || check<32>(edge)) return 1;
     return 0;
 }
 """
@@ -51,7 +51,11 @@ def test_part_layouts(tmp_path):
 
 # (instances in SM counts, more instances, horizons that are repeated over the batch)
 SIZES = [(0, 1, [64]), (0, 5, [2, 3, 4, 15, 63]), (0, 9, [2, 3, 5, 7, 15, 16, 17, 18, 64]), (1, 0, [70, 9, 33]),
-         (1, 1, [2, 3, 4, 5, 6, 7, 8, 9, 31]), (2, 0, [2, 7, 8, 65]), (2, 1, [2, 3, 4, 5, 6, 17, 40])]
+         (1, 1, [2, 3, 4, 5, 6, 7, 8, 9, 31]), (2, 0, [2, 7, 8, 65]), (2, 1, [2, 3, 4, 5, 6, 17, 40]),
+         # one instance at the edges of 4, 8, 16 and 32 parts; batches on clusters of 8, 4 and 2 CTAs, and just above
+         (0, 1, [23]), (0, 1, [24]), (0, 1, [47]), (0, 1, [48]), (0, 1, [255]), (0, 1, [256]), (0, 1, [511]),
+         (0, 12, [300, 2, 3, 31, 62, 63, 64, 65, 17, 5]), (0, 13, [256, 9, 2]), (0, 32, [48, 2, 3, 15, 30, 31, 32, 33]),
+         (0, 33, [48, 2, 3, 14, 15, 16, 17]), (0, 74, [50, 2, 5, 15, 16, 29]), (0, 75, [50, 2, 5, 15, 16, 29])]
 
 
 @pytest.mark.gpu
