@@ -660,11 +660,11 @@ def main():
     one_step()
     sv.set_profiling(False)
     phases = sv.phase_stats(reset=True)
-    # kernels per timed step of the graph: the prologue (init, G's weight-only entries, merit, accept),
-    # then per SQP iteration (as many as the profiled step's KKT launches) the six phase kernels once
+    # kernels per timed step of the graph: the prologue (init, merit, accept and, where the Schur complement reads
+    # G, its weight-only entries), then per SQP iteration (as many as the profiled step's KKT launches) the six phase kernels once
     # per part-batch branch and the while loop's control kernel
     branches = min(args.sqp_graph, B) if args.sqp_graph >= 2 else 1
-    launches_per_step = 4 + phases["kkt"][1] * (6 * branches + 1)
+    launches_per_step = (3 if args.pcg_precond == 1 else 4) + phases["kkt"][1] * (6 * branches + 1)
     total_ms = sum(step_ms)
     total_ms = shard.max_over_ranks(total_ms, device="cuda")
     ms_per_step = total_ms / args.steps
@@ -832,7 +832,7 @@ def main():
     peak = mp["hbm_gbs"] if mp else 6650.0
     pcg_kernel = ("pcg_cluster_kernel" if args.pcg_precond == 0 else
                   "pcg_pair_kernel" if tuned_cs == gpt.PCG_WARP_PAIR else
-                  "pcg_quad_kernel" if tuned_cs == gpt.PCG_WARP_QUAD else "pcg_chain_kernel")
+                  "pcg_part_kernel" if tuned_cs in (0, gpt.PCG_WARP_QUAD) else "pcg_chain_kernel")
     per_launch_bytes = (PCG_BJ_BYTES_PER_KNOT if args.pcg_precond == 0 else PCG_BYTES_PER_KNOT) * N * B
     per_launch_s = (pcg_ms / max(pcg_launches, 1)) / 1000.0
     achieved = per_launch_bytes / per_launch_s / 1e9 if per_launch_s > 0 else 0.0

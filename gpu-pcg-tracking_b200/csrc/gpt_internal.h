@@ -78,7 +78,7 @@ int part_variant(int B, int max_n, int num_sms);
 // whether a batch's KKT formation (KKT_G_NONE) takes one knot per lane
 bool kkt_lane(int total_knots, int max_n);
 // lambda64 (optional) replaces lambda when given; Ginv64c (optional): the compact inverses of
-// launch_schur64 (GC64 doubles per knot), with Ginv64 holding only the blocks its flags name
+// launch_schur64 (GC64 doubles per knot), which then replace Ginv and Ginv64
 cudaError_t launch_dz(const BatchView &bv, const float *Ginv, const double *Ginv64, const double *Ginv64c,
                       const float *C, const float *g, const float *lambda, const double *lambda64, float *dz,
                       int num_sms, cudaStream_t s, int ctas_per_sm = 16);

@@ -19,18 +19,21 @@ constexpr int DZ_WARPS = 4;
 // dz from lambda (FP32 or, when lambda64 is given, FP64).  The right-hand sides
 // q_k - lambda_k - (-A_k)^T lambda_{k+1} and r_k - (-B_k)^T lambda_{k+1} cancel
 // heavily, so they are accumulated in FP64 before the inverses apply.  Every input of a
-// knot is loaded in one batch (the kernel is bound by load latency) and staged in shared memory.
+// knot is loaded in one batch and staged in shared memory; lane i < 21 then forms row i of both products, without
+// divergence (the rows of C and the diagonals of the compact inverses follow on from each other).
 // COMPACT: the inverses come as launch_schur64's compact blocks (GC64 doubles per knot: the position
-// block, the velocity and control diagonals -- a quarter of the full layout's bytes); a block its
-// flags mark as not (block) diagonal is read from the full layout instead.  The sums are those of
-// the full layout term by term (the skipped terms are exact zeros).
+// block, the velocity and control diagonals -- a quarter of the full layout's bytes).  The sums are those of
+// the full layout term by term (the skipped terms are exact zeros).  512 x 128 knots: 43 us with a branch for
+// the states and one for the controls, 36 this way (129 MB, 20 us; now
+// the L1 pipe is 72 % busy); loading a knot ahead of the previous one's
+// arithmetic gave nothing.
 template <bool COMPACT>
-struct DzWarpSmem {
-    double gi[COMPACT ? GC64 : G_STRIDE];  // (Q + rho I)^{-1}, (R + rho I)^{-1}
-    double lv[2 * NS];                     // lambda_k, lambda_{k+1}
-    double s[NX];
-    float cm[C_STRIDE];  // -A_k, -B_k
-    float gv[NX];
+struct __align__(16) DzWarpSmem {
+    double gi[COMPACT ? GC64 : G_STRIDE + 1];  // (Q + rho I)^{-1}, (R + rho I)^{-1}
+    double lv[2 * NS];                         // lambda_k, lambda_{k+1}
+    double s[NX + 1];
+    float cm[C_STRIDE + 2];  // -A_k, -B_k
+    float gv[NX + 3];
 };
 
 template <bool COMPACT>
@@ -44,6 +47,7 @@ __global__ void __launch_bounds__(32 * DZ_WARPS)
     DzWarpSmem<COMPACT> &sm = sm_all[threadIdx.x >> 5];
     const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
+    const int row = lane < NX ? lane : 0;
     constexpr int GIN = COMPACT ? GC64 : G_STRIDE;
     for (int j = bv.j0 + gw; j < bv.j0 + bv.total_knots; j += nw) {
         const int b = bv.inst(j);
@@ -51,7 +55,7 @@ __global__ void __launch_bounds__(32 * DZ_WARPS)
         const int N = bv.N(b), k = j - bv.off(b);
         const bool last = (k == N - 1);
         const float *Cj = Cm + (size_t)C_STRIDE * j;
-        const int nl = last ? NS : 2 * NS;
+        const int nl = last ? NS : 2 * NS, nrows = last ? NS : NX;
         // ---- all loads of the knot, then the shared-memory stores
         constexpr int NGI = (GIN + 31) / 32, NCM = (C_STRIDE + 31) / 32;
         // the last knot's block has no R part (buffers of 245N - 49)
@@ -75,7 +79,7 @@ __global__ void __launch_bounds__(32 * DZ_WARPS)
         double lvv = 0.0;
         if (lane < nl) lvv = lambda64 ? lambda64[(size_t)NS * j + lane] : (double)lambda[(size_t)NS * j + lane];
         float gvv = 0.f;
-        if (lane < NX && (lane < NS || !last)) gvv = g[(size_t)NX * j + lane];
+        if (lane < nrows) gvv = g[(size_t)NX * j + lane];
 #pragma unroll
         for (int i = 0; i < NGI; ++i) {
             const int e = lane + 32 * i;
@@ -89,52 +93,42 @@ __global__ void __launch_bounds__(32 * DZ_WARPS)
         if (lane < 2 * NS) sm.lv[lane] = lvv;
         if (lane < NX) sm.gv[lane] = gvv;
         __syncwarp();
-        if (lane < NS) {
-            // q_k - (lambda_k + (-A_k)^T lambda_{k+1})
+        {
+            // states: q_k - (lambda_k + (-A_k)^T lambda_{k+1}); controls: r_k - (-B_k)^T lambda_{k+1}
             double a = 0.0;
             if (!last) {
+                const float2 *cr = reinterpret_cast<const float2 *>(sm.cm + NS * row);
+                const double2 *ln = reinterpret_cast<const double2 *>(sm.lv + NS);
 #pragma unroll
-                for (int t = 0; t < NS; ++t) a = fma((double)sm.cm[lane * NS + t], sm.lv[NS + t], a);
+                for (int t = 0; t < NS / 2; ++t) {
+                    const float2 c2 = cr[t];
+                    const double2 l2 = ln[t];
+                    a = fma((double)c2.x, l2.x, a);
+                    a = fma((double)c2.y, l2.y, a);
+                }
             }
-            sm.s[lane] = (double)sm.gv[lane] - (sm.lv[lane] + a);
-        } else if (lane < NX && !last) {
-            // r_k - (-B_k)^T lambda_{k+1}
-            const int i = lane - NS;
-            double a = 0.0;
-#pragma unroll
-            for (int t = 0; t < NS; ++t) a = fma((double)sm.cm[SS + i * NS + t], sm.lv[NS + t], a);
-            sm.s[lane] = (double)sm.gv[lane] - a;
+            if (lane < NS) a = sm.lv[row] + a;
+            if (lane < NX) sm.s[lane] = (double)sm.gv[lane] - a;
         }
         __syncwarp();
-        const int flags = COMPACT ? (int)sm.gi[0] : 0;
-        const double *full = COMPACT ? Ginv64 + (size_t)G_STRIDE * j : nullptr;  // the flagged blocks
-        if (lane < NS) {
-            double a = 0.0;
-            if (!COMPACT) {
-#pragma unroll
-                for (int t = 0; t < NS; ++t) a = fma(sm.gi[lane + NS * t], sm.s[t], a);
-            } else if (flags & 1) {
-                for (int t = 0; t < NS; ++t) a = fma(full[lane + NS * t], sm.s[t], a);
-            } else if (lane < NC) {
+        double a = 0.0;
+        if (COMPACT) {
+            if (lane < NC) {
 #pragma unroll
                 for (int t = 0; t < NC; ++t) a = fma(sm.gi[GC_POS + lane + NC * t], sm.s[t], a);
             } else {
-                a = sm.gi[GC_VEL + lane - NC] * sm.s[lane];
+                static_assert(GC_CTL == GC_VEL + NC, "the two diagonals");
+                a = sm.gi[GC_VEL + row - NC] * sm.s[row];
             }
-            dz[(size_t)NX * j + lane] = (float)a;
-        } else if (lane < NX && !last) {
-            const int i = lane - NS;
-            double a = 0.0;
-            if (!COMPACT) {
+        } else if (lane < NS) {
 #pragma unroll
-                for (int t = 0; t < NC; ++t) a = fma(sm.gi[SS + i + NC * t], sm.s[NS + t], a);
-            } else if (flags & 2) {
-                for (int t = 0; t < NC; ++t) a = fma(full[SS + i + NC * t], sm.s[NS + t], a);
-            } else {
-                a = sm.gi[GC_CTL + i] * sm.s[lane];
-            }
-            dz[(size_t)NX * j + lane] = (float)a;
+            for (int t = 0; t < NS; ++t) a = fma(sm.gi[lane + NS * t], sm.s[t], a);
+        } else if (lane < nrows) {
+            const int i = lane - NS;
+#pragma unroll
+            for (int t = 0; t < NC; ++t) a = fma(sm.gi[SS + i + NC * t], sm.s[NS + t], a);
         }
+        if (lane < nrows) dz[(size_t)NX * j + lane] = (float)a;
         __syncwarp();
     }
 }
@@ -144,7 +138,6 @@ cudaError_t launch_dz(const BatchView &bv, const float *Ginv, const double *Ginv
                       int num_sms, cudaStream_t s, int ctas_per_sm)
 {
     if (bv.total_knots <= 0) return cudaSuccess;
-    if (Ginv64c && !Ginv64) return cudaErrorInvalidValue;
     int blocks = (bv.total_knots + DZ_WARPS - 1) / DZ_WARPS;
     if (blocks > num_sms * ctas_per_sm) blocks = num_sms * ctas_per_sm;
     if (Ginv64c)
@@ -276,7 +269,7 @@ cudaError_t launch_merit(const BatchView &bv, const ProblemParams &P, int n_alph
 // merit reduction + accept
 // ------------------------------------------------------------------------
 
-constexpr int ACC_THREADS = 256;
+constexpr int ACC_THREADS = 256;  // the threads that sum (the others of a larger CTA only move the step)
 
 // Fixed-order sum of knot_merit[8 (kb + k) + a] over k for a < NA; result in out[a] (all threads).  A
 // thread loads its knots' NA merits together (two 16-byte loads for the 8 step sizes) and keeps NA
@@ -289,7 +282,7 @@ __device__ __forceinline__ void merit_sums(const float *km, int kb, int N, float
     double v[NA];
 #pragma unroll
     for (int a = 0; a < NA; ++a) v[a] = 0.0;
-    for (int k = tid; k < N; k += ACC_THREADS) {
+    for (int k = tid; tid < ACC_THREADS && k < N; k += ACC_THREADS) {
         const float *row = km + (size_t)NUM_ALPHAS * (kb + k);
         if constexpr (NA == NUM_ALPHAS) {
             const float4 lo = *reinterpret_cast<const float4 *>(row), hi = *reinterpret_cast<const float4 *>(row + 4);
@@ -303,6 +296,7 @@ __device__ __forceinline__ void merit_sums(const float *km, int kb, int N, float
     }
 #pragma unroll
     for (int a = 0; a < NA; ++a) {
+        if (warp >= NW) break;
         const double w = warp_sum(v[a]);
         if (lane == 0) scratch[a * NW + warp] = w;
     }
@@ -320,7 +314,11 @@ __device__ __forceinline__ void merit_sums(const float *km, int kb, int N, float
 
 // mode 0: initial merit of the iterate (merit0, toplevel.cuh:235-244)
 // mode 1: line-search decision and step (toplevel.cuh:384-444)
-__global__ void __launch_bounds__(ACC_THREADS)
+// mode 2: merits_out only
+// A chain of latencies (merits, state, decision, step) on one CTA per instance: the state and the thread's first KEEP
+// entries of xu and dz are loaded before the sums need their barriers.
+template <int NT, int KEEP>
+__global__ void __launch_bounds__(NT)
     accept_kernel(BatchView bv, int mode, SolverParams SP, const float *__restrict__ knot_merit,
                   const float *__restrict__ dz, float *__restrict__ xu, float *__restrict__ merits_out,
                   uint32_t *__restrict__ active_count)
@@ -330,6 +328,21 @@ __global__ void __launch_bounds__(ACC_THREADS)
     for (int b = bv.b0 + blockIdx.x; b < bv.b0 + bv.B; b += gridDim.x) {
         if (!bv.active(b)) continue;
         const int N = bv.N(b), kb = bv.off(b);
+        const int len = mode == 1 ? NX * N - NC : 0;
+        float *xb = xu + (size_t)NX * kb;
+        const float *db = dz + (size_t)NX * kb;
+        float xk[KEEP], dk[KEEP];
+#pragma unroll
+        for (int i = 0; i < KEEP; ++i) {
+            const int e = threadIdx.x + NT * i;
+            xk[i] = dk[i] = 0.f;
+            if (e < len) {
+                xk[i] = xb[e];
+                dk[i] = db[e];
+            }
+        }
+        InstState s = {};
+        if (threadIdx.x == 0 && bv.st) s = bv.st[b];
         float m[NUM_ALPHAS];
         if (mode == 0) {
             float m0[1];
@@ -347,7 +360,6 @@ __global__ void __launch_bounds__(ACC_THREADS)
                     if (mode != 0 || a == 0) merits_out[NUM_ALPHAS * b + a] = m[a];
             }
             if (bv.st) {
-                InstState &s = bv.st[b];
                 if (mode == 0) {
                     s.merit0 = m[0];
                     s.merit_init = m[0];
@@ -355,6 +367,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
                 } else {
                     float minm = s.merit0;
                     int best = 0;
+#pragma unroll
                     for (int a = 0; a < NUM_ALPHAS; ++a)
                         if (m[a] < minm) { minm = m[a]; best = a; }
                     const float f = SP.rho_factor;
@@ -382,6 +395,7 @@ __global__ void __launch_bounds__(ACC_THREADS)
                     // a failed factorisation or a non-finite reduction leaves no usable iterate
                     if (s.exit_flags & (GPT_EXIT_NONFINITE | GPT_EXIT_FACTOR)) s.active = 0;
                 }
+                bv.st[b] = s;
                 if (active_count && s.active) atomicAdd(active_count, 1u);
             }
             s_alpha = alpha;
@@ -389,10 +403,11 @@ __global__ void __launch_bounds__(ACC_THREADS)
         __syncthreads();
         const float alpha = s_alpha;
         if (alpha != 0.f) {
-            const int len = NX * N - NC;
-            float *xb = xu + (size_t)NX * kb;
-            const float *db = dz + (size_t)NX * kb;
-            for (int i = threadIdx.x; i < len; i += ACC_THREADS) xb[i] = fmaf(alpha, db[i], xb[i]);
+#pragma unroll
+            for (int i = 0; i < KEEP; ++i)
+                if (threadIdx.x + NT * i < len) xb[threadIdx.x + NT * i] = fmaf(alpha, dk[i], xk[i]);
+#pragma unroll 4
+            for (int i = threadIdx.x + NT * KEEP; i < len; i += NT) xb[i] = fmaf(alpha, db[i], xb[i]);
         }
         __syncthreads();
     }
@@ -405,7 +420,12 @@ cudaError_t launch_accept(const BatchView &bv, int mode, const SolverParams &SP,
     if (bv.B <= 0) return cudaSuccess;
     int blocks = bv.B;
     if (blocks > num_sms * 8) blocks = num_sms * 8;
-    accept_kernel<<<blocks, ACC_THREADS, 0, s>>>(bv, mode, SP, knot_merit, dz, xu, merits_out, active_count);
+    // long horizons of a few instances: more threads, so that the step is loaded ahead (1 x 511: 17 -> 9 us)
+    if (mode == 1 && bv.B <= num_sms && bv.total_knots > 128 * bv.B)
+        accept_kernel<512, 21><<<blocks, 512, 0, s>>>(bv, mode, SP, knot_merit, dz, xu, merits_out, active_count);
+    else
+        accept_kernel<ACC_THREADS, 12><<<blocks, ACC_THREADS, 0, s>>>(bv, mode, SP, knot_merit, dz, xu, merits_out,
+                                                                  active_count);
     return cudaGetLastError();
 }
 

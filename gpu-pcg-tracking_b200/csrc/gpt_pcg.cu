@@ -1818,8 +1818,8 @@ cudaError_t launch_pcg(const BatchView &bv, int max_n_knots, int min_n_knots, in
     if (max_n_knots > MAX_PCG_KNOTS) return cudaErrorInvalidValue;
     // The library's choice for packed rows and the exact preconditioner is the partitioned kernel: at every size
     // measured it is the fastest of the exact ones (us per launch, partitioned / one cyclic-reduction CTA: 1 x 32
-    // 33 / 68, 11 x 77 56 / 144, 512 x 128 191 / 781; horizons past 128 knots, which cyclic reduction spreads
-    // over CTAs that iterate: 1 x 511 246 / 6167).  Rows in the reference's layout keep cyclic reduction below.
+    // 27 / 68, 11 x 77 42 / 144, 512 x 128 187 / 781; horizons past 128 knots, which cyclic reduction spreads
+    // over CTAs that iterate: 1 x 511 85 / 6167).  Rows in the reference's layout keep cyclic reduction below.
     if (cluster_size == PCG_WARP_QUAD || (cluster_size == 0 && precond == 1 && fmt != 0)) {
         if (precond != 1 || fmt == 0) return cudaErrorInvalidValue;  // packed rows, exact preconditioner
         return launch_pcg_part(bv, max_n_knots, fmt, S, gamma, gamma64, lambda, lambda64, cr_ws, max_iter, tol,

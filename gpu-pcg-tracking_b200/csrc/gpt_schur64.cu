@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(32 * S64_WARPS, 5)
                 o[GC_VEL + m] = rv;
                 o[GC_CTL + m] = rc;
             } else {
-                o[0] = 0.0;  // flags: block diagonal
+                o[0] = 0.0;
                 if (!ok && bv.active(b)) atomicOr(&bv.st[b].exit_flags, GPT_EXIT_FACTOR);
             }
         }
