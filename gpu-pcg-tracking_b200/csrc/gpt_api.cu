@@ -124,7 +124,7 @@ struct gpt_handle {
     double *lam64 = nullptr;   // FP64 multipliers from the PCG, consumed by dz
     double *Ginv64 = nullptr;  // FP64 inverses (Q + rho I)^-1, (R + rho I)^-1 from Schur, consumed by dz
     double *Ginv64c = nullptr; // the same in compact form (GC64 doubles per knot) from the FP64 Schur kernel
-    double *crw = nullptr;     // FP64 cyclic-reduction couplings of the PCG preconditioner, 196 per knot
+    double *crw = nullptr;     // FP64 workspace of the exact PCG preconditioners, 392 per knot
     // adjoint workspace: right-hand side, its zero constraint part, gamma, multipliers, mu_z, partials
     float *adj_h = nullptr, *adj_zero = nullptr, *adj_gamma = nullptr, *adj_lam = nullptr, *adj_mu = nullptr,
           *adj_part = nullptr;
@@ -575,7 +575,7 @@ gpt_status gpt_pcg(gpt_handle *h, uint32_t N, const float *d_S, const float *d_P
                             h->pcg_out, nullptr, 0, (int)h->sc.pcg_cluster_size, h->num_sms, s));
     } else if (h->sc.pcg_cluster_size == 0 && h->sc.pcg_precond == 1) {
         // the library's choice: the partitioned kernel on the same conversion, from the caller's lambda (N = 100:
-        // 130 -> 75 us against cyclic reduction on the caller's rows)
+        // 130 -> 42 us against cyclic reduction on the caller's rows)
         GPT_CUDA(launch_pack_rows64((int)N, d_S, d_gamma, h->S64, h->gamma64, h->num_sms, s));
         GPT_CUDA(launch_pcg_part(single_view(N), (int)N, 2, h->S64, d_gamma, h->gamma64, d_lambda, d_lambda64, h->crw,
                                  (int)max_iter, tol, (int)exit_mode, h->pcg_out, nullptr, 0, h->num_sms, s, true));

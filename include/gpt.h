@@ -84,9 +84,9 @@ typedef struct gpt_solver_config {
     float rho_max;             /* RHO_MAX */
     float rho_min;             /* RHO_MIN */
     uint32_t pcg_cluster_size; /* CTAs per instance in the PCG (1,2,4,8,16); GPT_PCG_WARP_PAIR / GPT_PCG_WARP_QUAD:
-                                  one CTA per instance, factorisation from both ends / in parts (pcg_precond 1
-                                  only); 0 = chosen by the library (gpt_autotune's choice for the batch shape, else
-                                  1 ... 16) */
+                                  factorisation from both ends / in parts (pcg_precond 1 only); 0 = chosen by the
+                                  library (gpt_autotune's choice for the batch shape, else GPT_PCG_WARP_QUAD with
+                                  pcg_precond 1 and 1 ... 16 otherwise) */
     uint32_t pcg_precond;      /* 0: block-Jacobi Pinv (the reference's, oldschur.cuh:926-933);
                                   1 (default): exact block-tridiagonal LDL^T of each CTA's chunk of knots */
     uint32_t schur_fp64;       /* SQP loop and adjoint with pcg_precond 1: 1 (default) forms and stores the
@@ -120,12 +120,12 @@ typedef struct gpt_sqp_stats {
  * concurrently; same iteration and preconditioner (exact inverse of S) as pcg_cluster_size 1. */
 #define GPT_PCG_WARP_PAIR 32u
 
-/* pcg_cluster_size value: the PCG of one instance in one CTA whose warps each factor a part of the horizon
- * (partitioned block LDL^T: separator knots between the parts, whose reduced system one warp factors), with
- * 8, 4 or 2 warps by the batch size and the longest horizon of the call (few instances: more warps, a
- * shorter chain; many: less work); same iteration and preconditioner (exact inverse of S) as
+/* pcg_cluster_size value: the PCG of one instance by warps that each factor a part of the horizon
+ * (partitioned block LDL^T: separator knots between the parts, whose reduced system two warps factor from both
+ * ends), 2 to 32 of them on one CTA or a cluster of 2, 4 or 8, by the batch size and the longest horizon of the
+ * call (few instances: more parts, a shorter chain; many: less work); same iteration and preconditioner (exact inverse of S) as
  * pcg_cluster_size 1.  The same batch gives the same bits; an instance's last bits may differ between
- * batches that run with another number of warps. */
+ * batches that run with another number of parts. */
 #define GPT_PCG_WARP_QUAD 64u
 
 /* Default configs: the reference's logged experiment settings (dt 1/64, Euler,
@@ -390,7 +390,7 @@ gpt_status gpt_prep_csr(uint32_t knot_points, int32_t *h_col_ptr, int32_t *h_row
  * solves S lambda = gamma from the warm start in d_lambda (updated in place,
  * FP32).  d_lambda64 (optional, 14N doubles) receives the FP64 iterate; at
  * N >= ~64 only it can carry a relative residual near 1e-5.  With
- * pcg_cluster_size GPT_PCG_WARP_PAIR, S and gamma are first converted (exactly)
+ * pcg_precond 1 and pcg_cluster_size 0, GPT_PCG_WARP_PAIR or GPT_PCG_WARP_QUAD, S and gamma are first converted (exactly)
  * to FP64 packed rows in the handle's workspace. */
 gpt_status gpt_pcg(gpt_handle *h, uint32_t knot_points, const float *d_S, const float *d_Pinv,
                    const float *d_gamma, float *d_lambda, double *d_lambda64, uint32_t max_iter, float exit_tol,
