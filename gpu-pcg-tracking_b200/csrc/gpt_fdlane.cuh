@@ -187,7 +187,7 @@ __device__ __forceinline__ void crf2_add(const f2 *a, const f2 *na, const f2 *b,
 }
 
 // Columns 2p, 2p + 1 of the mass matrix, all rows (inverse dynamics at rest with a unit acceleration of the joint),
-// into sm.Minv
+// into M[row + 7 column][lane]
 template <int K>
 __device__ __forceinline__ void fl_mcol_fwd(const JointTrig &t, int j, f2 (&a)[6], f2 (&f)[model::NJ][6])
 {
@@ -214,7 +214,7 @@ __device__ __forceinline__ void fl_force_bwd(const JointTrig &t, f2 (&f)[model::
         fl_force_bwd<K - 1>(t, f);
     }
 }
-__device__ __forceinline__ void fl_mass_matrix(const JointTrig &t, FdLaneSmem &sm, int lane)
+__device__ __forceinline__ void fl_mass_matrix(const JointTrig &t, float (*M)[32], int lane)
 {
 #pragma unroll 1
     for (int j = 0; j < NQ; j += 2) {
@@ -227,8 +227,8 @@ __device__ __forceinline__ void fl_mass_matrix(const JointTrig &t, FdLaneSmem &s
         for (int k = 0; k < NQ; ++k) {
             float lo, hi;
             un2(f[k][2], lo, hi);
-            sm.Minv[k + NQ * j][lane] = lo;
-            if (j + 1 < NQ) sm.Minv[k + NQ * (j + 1)][lane] = hi;
+            M[k + NQ * j][lane] = lo;
+            if (j + 1 < NQ) M[k + NQ * (j + 1)][lane] = hi;
         }
     }
 }
@@ -393,6 +393,44 @@ __device__ __forceinline__ void fl_directions(const JointTrig &t, const float (&
     }
 }
 
+// qdd = M^{-1} (u - c) alone: the FP64 L D L^T of M's symmetric part, without pivoting (M is positive definite)
+__device__ __forceinline__ void fd_lane(const JointTrig &t, const float (&qd)[NQ], const float (&u)[NC], float (&qdd)[NQ],
+                                        float (*M)[32], int lane)
+{
+    double A[NQ][NQ], x[NQ], rd[NQ];
+    {
+        float zero[NQ], c[NQ];
+#pragma unroll
+        for (int i = 0; i < NQ; ++i) zero[i] = 0.f;
+        fl_mass_matrix(t, M, lane);
+        rnea<false>(t, qd, zero, -1, -1, c, nullptr);
+#pragma unroll
+        for (int j = 0; j < NQ; ++j) {
+#pragma unroll
+            for (int r = j; r < NQ; ++r) A[j][r] = 0.5 * ((double)M[r + NQ * j][lane] + (double)M[j + NQ * r][lane]);
+            x[j] = (double)u[j] - (double)c[j];
+        }
+    }
+#pragma unroll
+    for (int p = 0; p < NQ; ++p) {
+        rd[p] = rcp_newton(A[p][p]);
+#pragma unroll
+        for (int i = p + 1; i < NQ; ++i) {
+            const double l = A[p][i] * rd[p];
+            x[i] = fma(-l, x[p], x[i]);
+#pragma unroll
+            for (int r = i; r < NQ; ++r) A[i][r] = fma(-l, A[p][r], A[i][r]);
+        }
+    }
+#pragma unroll
+    for (int p = NQ - 1; p >= 0; --p) {
+#pragma unroll
+        for (int i = p + 1; i < NQ; ++i) x[p] = fma(-A[p][i], x[i], x[p]);
+        x[p] *= rd[p];
+        qdd[p] = (float)x[p];
+    }
+}
+
 // qdd = M^{-1} (u - c) and the columns of df/du = [-M^{-1} dID/dq, -M^{-1} dID/dqd, M^{-1}] at (q, qd, u), each handed to
 // emit(FdBlock<i>(), column of the block, values[7]) by every lane at the same time
 template <class Emit>
@@ -406,7 +444,7 @@ __device__ __forceinline__ void fd_gradient_lane(const JointTrig &t, const float
             float zero[NQ], c[NQ];
 #pragma unroll
             for (int i = 0; i < NQ; ++i) zero[i] = 0.f;
-            fl_mass_matrix(t, sm, lane);
+            fl_mass_matrix(t, sm.Minv, lane);
             rnea<false>(t, qd, zero, -1, -1, c, nullptr);
 #pragma unroll
             for (int j = 0; j < NQ; ++j) {

@@ -5,10 +5,10 @@
 //                   pitch / yaw per row, one thread per row (generateeepos.cu:101-107 launches it
 //                   once per trajectory row)
 //   fd_kernel       forward_dynamics (:4351-4395): qdd = M^{-1}(u - c(q, qd)), gravity 0, one group
-//                   of 8 lanes per row (fd_group)
+//                   of 8 lanes per row (fd_group); fd_lane_kernel one lane per row
 //   fd_grad_kernel  forwardDynamicsAndGradient (rbdfiles/iiwa_eepos_plant.cuh:130-160): qdd and
 //                   df/du = [-M^{-1} dID/dq, -M^{-1} dID/dqd, M^{-1}] (7 x 21, column-major), one
-//                   half-warp per row with the lane roles of kkt_kernel
+//                   half-warp per row with the lane roles of kkt_kernel; fd_grad_lane_kernel one lane per row
 //
 // Rows are read with a caller-given stride, so the rows of a trajectory (21 floats: x, u) and plain
 // states (14 floats) are both accepted.
@@ -213,9 +213,47 @@ cudaError_t launch_ee_pose(uint32_t n, const float *x, uint32_t stride, float *p
     return cudaGetLastError();
 }
 
+// Forward dynamics with one row per lane (gpt_fdlane.cuh): the mass matrix two columns at a time in packed FP32, the FP64
+// solve in registers.  200,003 rows: 24.6 us against 78 with eight lanes per row, one of which each evaluates a column
+// (the rows' 112 bytes take 3.5 us; bound by issue).
+constexpr int FDL_WARPS = 4;
+
+__global__ void __launch_bounds__(32 * FDL_WARPS, 4)
+    fd_lane_kernel(uint32_t n, const float *__restrict__ xu, uint32_t stride, float *__restrict__ qdd_out)
+{
+    __shared__ struct {
+        float M[CC][32], out[NS * 34];
+    } sm_all[FDL_WARPS];
+    auto &sm = sm_all[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const size_t i0 = (size_t)blockIdx.x * blockDim.x + (threadIdx.x & ~31);
+    const bool valid = i0 + lane < n;  // lanes past the end follow the last row and store nothing
+    const uint32_t mask = __ballot_sync(0xffffffffu, valid);
+    const float *x = xu + (size_t)stride * (valid ? i0 + lane : n - 1);
+    float q[NQ], qd[NQ], u[NC], qdd[NQ];
+#pragma unroll
+    for (int i = 0; i < NQ; ++i) {
+        q[i] = x[i];
+        qd[i] = x[NQ + i];
+        u[i] = x[NS + i];
+    }
+    JointTrig t;
+    joint_trig(q, t);
+    fd_lane(t, qd, u, qdd, sm.M, lane);
+    store_rows<NQ, NQ>(sm.out, qdd, qdd_out + NQ * i0, mask, lane);
+}
+
 cudaError_t launch_fd(uint32_t n, const float *xu, uint32_t stride, float *qdd, cudaStream_t s)
 {
     if (n == 0) return cudaSuccess;
+    // up to 37,888 rows (four CTAs per SM) the lane form takes 8 us, launch included, the eight-lane form 8.4 at 4095 rows
+    // and 0.4 us more per 1,000
+    constexpr uint32_t FDL_MIN = 4096;
+    if (n >= FDL_MIN) {
+        constexpr int per = 32 * FDL_WARPS;
+        fd_lane_kernel<<<(unsigned)(((size_t)n + per - 1) / per), per, 0, s>>>(n, xu, stride, qdd);
+        return cudaGetLastError();
+    }
     fd_kernel<<<(unsigned)(((size_t)n * 8 + 127) / 128), 128, 0, s>>>(n, xu, stride, qdd);
     return cudaGetLastError();
 }

@@ -130,3 +130,28 @@ def test_forward_dynamics_gradient_by_row_count(gpt, oracle, golden, n, stride):
         for b in range(3):
             blk = slice(49 * b, 49 * (b + 1))
             assert np.abs(df[k, blk] - wdf[blk]).max() <= 1e-4 * max(1e-3, np.abs(wdf[blk]).max()), (k, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,stride", [(4095, 21), (4096, 21), (4097, 22), (4096 + 63, 24), (37888 + 33, 21)])
+def test_forward_dynamics_by_row_count(gpt, oracle, golden, n, stride):
+    """Both forms of the forward dynamics (eight lanes per row below 4096 rows, a lane per row from there on) against the
+    FP64 oracle with the tolerance used for the gradient's qdd; a row of NaN stays alone, and nothing is written past the
+    last row."""
+    tr = np.concatenate([golden["traj_0_1"], golden["traj_3_4"]])
+    rng = np.random.default_rng(n)
+    x = np.zeros((n, stride), np.float32)
+    x[:, :21] = tr[rng.integers(0, len(tr), n), :21] + rng.uniform(-0.1, 0.1, (n, 21)).astype(np.float32)
+    bad = n // 2
+    x[bad, 3] = np.nan
+    xu, out = dev(x), torch.full((n + 3, 7), 7.0, device="cuda")
+    gpt._check(gpt.lib().gpt_forward_dynamics(n, gpt._ptr(xu), stride, gpt._ptr(out), gpt._stream(None)))
+    torch.cuda.synchronize()
+    qdd = out.cpu().numpy()
+    assert (qdd[n:] == 7.0).all() and np.isnan(qdd[bad]).all()
+    assert np.isfinite(qdd[:n][np.arange(n) != bad]).all()
+    check = np.unique(np.concatenate([np.arange(3), np.arange(n - 40, n), [bad - 1, bad + 1], rng.integers(0, n, 40)]))
+    for k in check[check != bad]:
+        row = x[k].astype(np.float64)
+        wq, _ = oracle.fd_grad(row[:7], row[7:14], row[14:21])
+        assert np.abs(qdd[k] - wq).max() <= 1e-5 * max(1.0, np.abs(wq).max()), k
