@@ -356,7 +356,10 @@ __global__ void __launch_bounds__(32 * KKTL_WARPS, 8 / KKTL_WARPS)
     const int j0 = bv.j0 + 32 * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5), jend = bv.j0 + bv.total_knots;
     const int j = min(j0 + lane, jend - 1), b = bv.inst(j), N = bv.N(b), k = j - bv.off(b);
     const bool live = j0 + lane < jend && bv.active(b), valid = live && k < N - 1;
-    if (!__syncthreads_or(valid)) return;  // converged instances only
+    // nothing to store: stopped instances, and last knots whose gradient the knot before writes (a last knot that
+    // writes its own, ref_terminal 0, can be the only live one of a CTA)
+    const bool grad_here = live && (valid || !P.ref_terminal);
+    if (!__syncthreads_or(grad_here)) return;
     const uint32_t mask = __ballot_sync(0xffffffffu, valid);
     const float *x = xu + (size_t)NX * j;
     float q[NQ], qd[NQ], u[NC], qdd[NQ];
@@ -383,7 +386,7 @@ __global__ void __launch_bounds__(32 * KKTL_WARPS, 8 / KKTL_WARPS)
         grad(gl[0], gl[1], gl[2], gv);
 #pragma unroll
         for (int i = 0; i < NC; ++i) gr[i] = P.r_cost * u[i];
-        const uint32_t states = __ballot_sync(0xffffffffu, live && (valid || !P.ref_terminal));
+        const uint32_t states = __ballot_sync(0xffffffffu, grad_here);
         store_rows<NS, NX>(sm.out, gv, g + (size_t)NX * j0, states, lane);
         store_rows<NC, NX>(sm.out, gr, g + (size_t)NX * j0 + NS, mask, lane);
         if (P.ref_terminal && valid && k == N - 2) {
