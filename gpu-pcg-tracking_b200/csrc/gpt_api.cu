@@ -1289,7 +1289,7 @@ gpt_status gpt_sqp_adjoint(gpt_handle *h, uint32_t B, const uint32_t *h_N, const
     GPT_CUDA(cudaMemsetAsync(h->adj_lam, 0, sizeof(float) * NS * T, s));
     GPT_CUDA(launch_pcg(bv, maxN, minN, fmt, (int)SP.pcg_precond, S_rows, nullptr, h->gamma, h->gamma64, h->adj_lam, h->lam64,
                         h->crw, (int)SP.pcg_max_iter, SP.pcg_tol, (int)SP.pcg_exit_mode, nullptr, nullptr, 0,
-                        (int)SP.pcg_cluster_size, ns, s));
+                        (int)SP.pcg_cluster_size, ns, s, true));
     GPT_CUDA(cudaMemsetAsync(h->dz, 0, sizeof(float) * NX * T, s));
     GPT_CUDA(launch_dz(bv, h->Ginv, h->Ginv64, f64 ? h->Ginv64c : nullptr, h->C, h->g, nullptr, h->lam64, h->dz, ns,
                        s));
@@ -1306,7 +1306,7 @@ gpt_status gpt_sqp_adjoint(gpt_handle *h, uint32_t B, const uint32_t *h_N, const
     GPT_CUDA(cudaMemsetAsync(h->adj_lam, 0, sizeof(float) * NS * T, s));
     GPT_CUDA(launch_pcg(bv, maxN, minN, fmt, (int)SP.pcg_precond, S_rows, nullptr, h->adj_gamma, h->adj_gamma64, h->adj_lam,
                         h->adj_lam64, h->crw, (int)SP.pcg_max_iter, SP.pcg_tol, (int)SP.pcg_exit_mode, nullptr,
-                        nullptr, 0, (int)SP.pcg_cluster_size, ns, s));
+                        nullptr, 0, (int)SP.pcg_cluster_size, ns, s, true));
     GPT_CUDA(cudaMemsetAsync(h->adj_mu, 0, sizeof(float) * NX * T, s));
     GPT_CUDA(launch_dz(bv, h->Ginv, h->Ginv64, f64 ? h->Ginv64c : nullptr, h->C, h->adj_h, nullptr, h->adj_lam64,
                        h->adj_mu, ns, s));
@@ -1437,7 +1437,7 @@ static gpt_status enqueue_track_adjoint(gpt_handle *h, const SqpPlan &pl, float 
     GPT_CUDA(cudaMemsetAsync(h->adj_lam, 0, sizeof(float) * NS * T, s));
     GPT_CUDA(launch_pcg(bv, pl.maxN, pl.minN, fmt, (int)SP.pcg_precond, S_rows, nullptr, h->gamma, h->gamma64,
                         h->adj_lam, h->lam64, h->crw, (int)SP.pcg_max_iter, SP.pcg_tol, (int)SP.pcg_exit_mode, nullptr,
-                        nullptr, 0, (int)SP.pcg_cluster_size, ns, s));
+                        nullptr, 0, (int)SP.pcg_cluster_size, ns, s, true));
     GPT_CUDA(cudaMemsetAsync(h->dz, 0, sizeof(float) * NX * T, s));
     GPT_CUDA(launch_dz(bv, h->Ginv, h->Ginv64, f64 ? h->Ginv64c : nullptr, h->C, h->g, nullptr, h->lam64, h->dz, ns,
                        s));
@@ -1453,7 +1453,7 @@ static gpt_status enqueue_track_adjoint(gpt_handle *h, const SqpPlan &pl, float 
     GPT_CUDA(cudaMemsetAsync(h->adj_lam, 0, sizeof(float) * NS * T, s));
     GPT_CUDA(launch_pcg(bv, pl.maxN, pl.minN, fmt, (int)SP.pcg_precond, S_rows, nullptr, h->adj_gamma,
                         h->adj_gamma64, h->adj_lam, h->adj_lam64, h->crw, (int)SP.pcg_max_iter, SP.pcg_tol,
-                        (int)SP.pcg_exit_mode, nullptr, nullptr, 0, (int)SP.pcg_cluster_size, ns, s));
+                        (int)SP.pcg_exit_mode, nullptr, nullptr, 0, (int)SP.pcg_cluster_size, ns, s, true));
     GPT_CUDA(cudaMemsetAsync(h->adj_mu, 0, sizeof(float) * NX * T, s));
     GPT_CUDA(launch_dz(bv, h->Ginv, h->Ginv64, f64 ? h->Ginv64c : nullptr, h->C, h->adj_h, nullptr, h->adj_lam64,
                        h->adj_mu, ns, s));

@@ -60,11 +60,12 @@ int pcg_pick_cluster(int maxN, int B, int num_sms, int requested);
 // coupling blocks; unused by precond 0)
 // fmt 0: reference 3-block rows (S, Pinv floats); 1: packed FP32 rows (PK); 2: packed FP64 rows (PK64,
 // S points at doubles) with FP64 gamma64 -- chain preconditioner only.  cluster_size PCG_WARP_PAIR runs
-// pcg_pair_kernel (precond 1, fmt 1 or 2; cr_ws holds its factors and FP64 vectors)
+// pcg_pair_kernel (precond 1, fmt 1 or 2; cr_ws holds its factors and FP64 vectors).  Starts from lambda (PCG_WARP_QUAD
+// by name from 0); zero_start: the caller says that lambda is 0
 cudaError_t launch_pcg(const BatchView &bv, int max_n_knots, int min_n_knots, int fmt, int precond, const float *S,
                        const float *Pinv, const float *gamma, const double *gamma64, float *lambda, double *lambda64,
                        double *cr_ws, int max_iter, float tol, int exit_mode, uint32_t *out_iters, uint32_t *pcg_log,
-                       int log_stride, int cluster_size, int num_sms, cudaStream_t s);
+                       int log_stride, int cluster_size, int num_sms, cudaStream_t s, bool zero_start = false);
 // the partitioned kernel of cluster_size PCG_WARP_QUAD (gpt_part.cu; fmt 1 or 2, exact preconditioner); warm:
 // start from lambda instead of 0
 cudaError_t launch_pcg_part(const BatchView &bv, int max_n, int fmt, const void *S, const float *gamma,

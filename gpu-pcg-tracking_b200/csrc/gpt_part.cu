@@ -2,9 +2,9 @@
 // instance, whose warps factor parts of the horizon.
 //
 // Solves S lambda = gamma by conjugate gradients with the exact inverse of S as the preconditioner
-// (z = S^{-1} r up to rounding), so the iteration stops after one step; it starts from lambda = 0
-// (r_0 = gamma: a warm start cannot save the one step) unless asked to start from the given lambda.  With M = -S (SPD), A_k = M_kk and
-// E_k = M_{k,k-1} = -L_k (L_k the left block of row k of S), the horizon is cut by P - 1 separator
+// (z = S^{-1} r up to rounding), so the iteration stops after one step, from any start.  It starts from lambda = 0
+// (r_0 = gamma); asked to start from the given lambda, it keeps one that meets the tolerance (warm).  With M = -S (SPD),
+// A_k = M_kk and E_k = M_{k,k-1} = -L_k (L_k the left block of row k of S), the horizon is cut by P - 1 separator
 // knots s_1 < ... < s_{P-1} into P parts.  Part 0 is eliminated top-down toward s_1 and part P-1
 // bottom-up toward s_{P-1}; a middle part top-down from its left to its right separator, which couples
 // the two.  The separators' block-tridiagonal system is eliminated by two warps from both ends, then every
@@ -66,6 +66,7 @@ constexpr int QLD = 20;                    // leading dimension of W and V (conf
 constexpr int QW_D = NS * QLD;             // W or V (14 rows x 16 columns)
 constexpr int QROWS_D = 2 * 2 * 37;        // pivot rows: 2 sets of 2 rows (D, E^T), 37 pairs apart
 constexpr int QBUF = QROWS_D + 2 * NS;     // pivot rows; B^{-1} by rows
+constexpr int RED_N = 4;                   // values of a reduction
 constexpr int RR_PERIOD = 32;              // CG iterations between true-residual replacements
 
 // A kernel variant: a cluster of CL CTAs of WC warps per instance (NW = CL WC parts, in order over the CTAs), SL staging
@@ -83,7 +84,7 @@ struct PartCfg {
     static constexpr int MID = MIDS * QW_D > SEP_SX + WC * NS ? MIDS * QW_D : SEP_SX + WC * NS;
     static size_t smem_bytes(int n)
     {
-        return sizeof(double) * (size_t)(NS * n + WC * (REGION + QBUF) + MID + 2 * NW * 3 + 4);
+        return sizeof(double) * (size_t)(NS * n + WC * (REGION + QBUF) + MID + 2 * NW * RED_N + 4);
     }
 };
 
@@ -340,9 +341,9 @@ struct PartSmem {
         stg = base;                         // per warp: staged rows / steps; the separators' blocks
         buf = stg + CF::WC * CF::REGION;    // per warp: pivot rows; the backward sweep's scratch
         wmid = buf + CF::WC * QBUF;
-        red = wmid + CF::MID;               // 2 sets x NW warps x 3
-        lay = reinterpret_cast<int *>(red + 2 * CF::NW * 3);  // parts, first separator, spacing, this CTA's knots
-        xv = red + 2 * CF::NW * 3 + 4;      // 14 n: y, then z, then x (of the CTA's knots and all separators)
+        red = wmid + CF::MID;               // 2 sets x NW warps x RED_N
+        lay = reinterpret_cast<int *>(red + 2 * CF::NW * RED_N);  // parts, first separator, spacing, this CTA's knots
+        xv = red + 2 * CF::NW * RED_N + 4;  // 14 n: y, then z, then x (of the CTA's knots and all separators)
     }
 };
 
@@ -495,7 +496,7 @@ struct PartArgs {
     const double *gamma64;
     float *lambda;
     double *lambda64, *ws;
-    int max_iter, exit_mode, log_stride, warm;
+    int max_iter, exit_mode, log_stride;
     float tol;
     uint32_t *out_iters, *pcg_log;
 };
@@ -529,9 +530,45 @@ struct PartCtx {
     }
 };
 
-// y in xv -> x of M x = y in xv, and S x in the workspace (QW_SX)
+// This lane's part of a lower bound of ||gamma - S lambda||^2 for the caller's lambda, by warp w of nw: the residual of one
+// knot (lane pair c its row c), and a NaN if an entry of lambda is not finite.
+// (Out of line: it would cost the elimination registers.)
 template <int FMT, class CF>
-__device__ __forceinline__ void part_apply(const PartArgs &A)
+__device__ __noinline__ double part_start_bound(const PartArgs &A, int w, int nw)
+{
+    using ST = typename PartRows<FMT>::ST;
+    constexpr ptrdiff_t ks = PartCtx<FMT, CF>::ks;
+    extern __shared__ __align__(16) double part_dyn_smem[];
+    const int *lay = PartSmem<CF>(part_dyn_smem).lay;
+    const PartCtx<FMT, CF> cx(A);
+    const int lo = lay[3], hi = lay[4];
+    const int lane = threadIdx.x & 31, c = lane >> 1, h = lane & 1, cl = c < NS ? c : NS - 1;
+    const float *lam = cx.A.lambda + NS * cx.kg0;
+    double s = 0.0;
+#pragma unroll 8
+    for (int e = NS * lo + 32 * w + lane; e < NS * hi; e += 32 * nw) s = fma(0.0, (double)lam[e], s);
+    const int k = lo + (hi - lo) * w / nw;
+    if (k >= hi) return s;
+    const bool left = k > 0, right = k < cx.n - 1;
+    const ST *row = cx.rows() + ks * k;
+    const float *x = lam + NS * k + h;
+    double a = 0.0, b = 0.0, d = 0.0;
+#pragma unroll
+    for (int q = 0; q < 7; ++q) {
+        const int j = 2 * q + h;
+        if (left) a = fma((double)row[cl + NS * j], (double)x[2 * q - NS], a);
+        b = fma((double)row[PK_LEFT_N + tri_idx(cl, j)], (double)x[2 * q], b);
+        if (right) d = fma((double)row[ks + j + NS * cl], (double)x[2 * q + NS], d);
+    }
+    a += b + d;
+    const double r = cx.gam(NS * k + cl) - (a + __shfl_xor_sync(0xffffffffu, a, 1));
+    return h == 0 && c < NS ? fma(r, r, s) : s;
+}
+
+// y in xv -> x of M x = y in xv, and S x in the workspace (QW_SX); WARM and check: bound as of part_start_bound, by the
+// warps that wait for the separators
+template <int FMT, class CF, bool WARM>
+__device__ __forceinline__ void part_apply(const PartArgs &A, bool check, double &bound)
 {
     using ST = typename PartRows<FMT>::ST;
     constexpr int NW = CF::NW;
@@ -654,6 +691,10 @@ __device__ __forceinline__ void part_apply(const PartArgs &A)
             }
         }
     }
+    if (WARM && check) {
+        const int w0 = rank == 0 && P >= 2 ? (NW == 2 ? 1 : 2) : 0;
+        if (warp >= w0) bound = part_start_bound<FMT, CF>(A, warp - w0, CF::WC - w0);
+    }
     part_sync<CF>();
     // ---- backward through every part, and S x with it: a staged step is L^{-1} of the knot it solves and a row
     // of S.  Top-down parts go through the rows r = right separator .. pa: t = L_r^T x_r, then x_{r-1}, then row r
@@ -772,22 +813,23 @@ __device__ __forceinline__ void part_apply(const PartArgs &A)
 }
 
 // sums of v[0 .. CNT-1] over the instance's threads, in a fixed order (set: alternate between calls)
-template <class CF, int CNT>
-__device__ __forceinline__ void part_sum(double (&v)[CNT], int set)
+template <class CF, int CNT, int LEN>
+__device__ __forceinline__ void part_sum(double (&v)[LEN], int set)
 {
+    static_assert(CNT <= LEN && CNT <= RED_N, "the reduction's slots");
     extern __shared__ __align__(16) double part_dyn_smem[];
-    double *red = PartSmem<CF>(part_dyn_smem).red + set * CF::NW * 3;
+    double *red = PartSmem<CF>(part_dyn_smem).red + set * CF::NW * RED_N;
     const int lane = threadIdx.x & 31, part = part_rank<CF>() * CF::WC + (threadIdx.x >> 5);
 #pragma unroll
     for (int q = 0; q < CNT; ++q) {
         const double s = warp_sum(v[q]);
-        if (lane < CF::CL) part_peer<CF>(red, lane)[3 * part + q] = s;
+        if (lane < CF::CL) part_peer<CF>(red, lane)[RED_N * part + q] = s;
     }
     part_sync<CF>();
 #pragma unroll
     for (int q = 0; q < CNT; ++q) {
         double s = 0.0;
-        for (int w = 0; w < CF::NW; ++w) s += red[3 * w + q];
+        for (int w = 0; w < CF::NW; ++w) s += red[RED_N * w + q];
         v[q] = s;
     }
 }
@@ -805,11 +847,16 @@ struct PartRange {
     }
 };
 
-// r = gamma - S lambda (the workspace's lambda) into the workspace and r . r; a rare path
+// r = gamma - S lambda (the workspace's lambda; given: the caller's, copied there first) into the workspace and r . r; a
+// rare path
 template <int FMT, class CF>
-__device__ __noinline__ double part_true_residual(const PartArgs &A, int set)
+__device__ __noinline__ double part_true_residual(const PartArgs &A, int set, bool given = false)
 {
     const PartCtx<FMT, CF> cx(A);
+    if (given) {
+        const PartRange<CF> rg;
+        for (int e = rg.first; e < rg.end; e += 32 * CF::WC) cx.vec(QW_LAM, e) = (double)A.lambda[NS * cx.kg0 + e];
+    }
     const typename PartRows<FMT>::ST *Sb = cx.rows();
     constexpr ptrdiff_t ks = PartCtx<FMT, CF>::ks;
     double s[1] = {0.0};
@@ -832,7 +879,9 @@ __device__ __noinline__ double part_true_residual(const PartArgs &A, int set)
     return s[0];
 }
 
-template <int FMT, class CF>
+// WARM: from the caller's lambda (a kernel of its own: the code for it costs the one that starts from 0 nine us of 187 at
+// 512 x 128)
+template <int FMT, class CF, bool WARM>
 __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const __grid_constant__ PartArgs A)
 {
     static_assert(FMT == 1 || FMT == 2, "packed rows only");
@@ -840,6 +889,11 @@ __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const _
     extern __shared__ __align__(16) double part_dyn_smem[];
     double *xv = PartSmem<CF>(part_dyn_smem).xv;
     const int tid = threadIdx.x;
+    // A given start that does not meet the tolerance leads to the solution from 0 too.  Whether it does is told by a part of
+    // its residual, formed by warps that wait for the separators, and by all of it only where that part does not exclude
+    // it: a residual ahead of the elimination took 3.6 us more a launch at 32 knots (27 us in all) and 62 at 512 x 128
+    // (187), the part takes 0 and 12.  The exit test on r . z, or no iteration at all, takes the start as it is.
+    const bool check = WARM && A.exit_mode == 0 && A.max_iter > 0;
     {
         const PartCtx<FMT, CF> cx(A);
         if (!A.bv.active(cx.inst)) return;  // (the whole cluster)
@@ -865,7 +919,7 @@ __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const _
     bool conv = false, bad = false, in_xv = false;
     bool has_res = false;  // r and lambda are in the workspace (before: r = gamma, lambda = 0)
     double eta = 0.0, gg = 0.0, alpha = 0.0;
-    if (A.warm) {
+    if (WARM && !check) {
         part_sync<CF>();
         const PartCtx<FMT, CF> cx(A);
         const PartRange<CF> rg;
@@ -890,10 +944,11 @@ __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const _
         return A.exit_mode == 0 ? (r2 <= (double)A.tol * (double)A.tol * gg) : (fabs(e) < (double)A.tol);
     };
     for (;;) {
-        part_apply<FMT, CF>(A);
+        double bound = 0.0;
+        part_apply<FMT, CF, WARM>(A, check && it == 0, bound);
         const PartCtx<FMT, CF> cx(A);
         const PartRange<CF> rg;
-        double dd[3] = {0.0, 0.0, 0.0};  // r . z, r . r with z = -x; x . S x
+        double dd[4] = {0.0, 0.0, 0.0, bound};  // r . z, r . r with z = -x; x . S x; the start's bound
         // the thread's first KEEP entries of r and S x stay in registers for the new residual's norm
         constexpr int KEEP = 8;
         double rk[KEEP], sk[KEEP];
@@ -916,11 +971,21 @@ __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const _
             if (rg.first + NT * i < rg.end) dots(rk[i], xv[rg.first + NT * i], sk[i]);
         for (int e = rg.first + NT * KEEP; e < rg.end; e += NT)
             dots(has_res ? cx.vec(QW_RES, e) : cx.gam(e), xv[e], cx.vec(QW_SX, e));
-        part_sum<CF, 3>(dd, set);
+        part_sum<CF, WARM ? 4 : 3>(dd, set);
         set ^= 1;
         if (it == 0) {
             if (!has_res) gg = dd[1];
-            conv = converged(dd[0], dd[1]);
+            conv = check ? gg == 0.0 : converged(dd[0], dd[1]);
+            if (check && !conv && !(dd[3] > (double)A.tol * (double)A.tol * gg)) {
+                const double r0 = part_true_residual<FMT, CF>(A, set, true);
+                set ^= 1;
+                bad = !isfinite(r0);
+                conv = converged(0.0, r0);
+                if (bad || conv) {
+                    has_res = true;  // the start is the result
+                    break;
+                }
+            }
         } else {
             if (!isfinite(dd[0])) {
                 bad = true;
@@ -1028,10 +1093,10 @@ __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const _
     }
 }
 
-template <int FMT, class CF>
+template <int FMT, class CF, bool WARM>
 static cudaError_t launch_part_t(const PartArgs &A, int max_n, cudaStream_t s)
 {
-    auto kern = pcg_part_kernel<FMT, CF>;
+    auto kern = pcg_part_kernel<FMT, CF, WARM>;
     const size_t smem = CF::smem_bytes(max_n);
     const cudaError_t e = ensure_func_attrs((const void *)kern, smem);
     if (e != cudaSuccess) return e;
@@ -1080,9 +1145,10 @@ int part_variant(int B, int max_n, int num_sms)
 }
 
 template <class CF>
-static cudaError_t launch_part_f(const PartArgs &A, int max_n, int fmt, cudaStream_t s)
+static cudaError_t launch_part_f(const PartArgs &A, int max_n, int fmt, bool warm, cudaStream_t s)
 {
-    return fmt == 2 ? launch_part_t<2, CF>(A, max_n, s) : launch_part_t<1, CF>(A, max_n, s);
+    if (warm) return fmt == 2 ? launch_part_t<2, CF, true>(A, max_n, s) : launch_part_t<1, CF, true>(A, max_n, s);
+    return fmt == 2 ? launch_part_t<2, CF, false>(A, max_n, s) : launch_part_t<1, CF, false>(A, max_n, s);
 }
 
 cudaError_t launch_pcg_part(const BatchView &bv, int max_n, int fmt, const void *S, const float *gamma,
@@ -1091,14 +1157,14 @@ cudaError_t launch_pcg_part(const BatchView &bv, int max_n, int fmt, const void 
                             int num_sms, cudaStream_t s, bool warm)
 {
     const PartArgs A{bv,       S,         gamma,      gamma64, lambda,    lambda64, ws,
-                     max_iter, exit_mode, log_stride, warm ? 1 : 0, tol, out_iters, pcg_log};
+                     max_iter, exit_mode, log_stride, tol, out_iters, pcg_log};
     switch (bv.part_variant ? bv.part_variant : part_variant(bv.B, max_n, num_sms)) {
-    case PART_32: return launch_part_f<Part32>(A, max_n, fmt, s);
-    case PART_16: return launch_part_f<Part16>(A, max_n, fmt, s);
-    case PART_8X2: return launch_part_f<Part8x2>(A, max_n, fmt, s);
-    case PART_8: return launch_part_f<Part8>(A, max_n, fmt, s);
-    case PART_4: return launch_part_f<Part4>(A, max_n, fmt, s);
-    default: return launch_part_f<Part2>(A, max_n, fmt, s);
+    case PART_32: return launch_part_f<Part32>(A, max_n, fmt, warm, s);
+    case PART_16: return launch_part_f<Part16>(A, max_n, fmt, warm, s);
+    case PART_8X2: return launch_part_f<Part8x2>(A, max_n, fmt, warm, s);
+    case PART_8: return launch_part_f<Part8>(A, max_n, fmt, warm, s);
+    case PART_4: return launch_part_f<Part4>(A, max_n, fmt, warm, s);
+    default: return launch_part_f<Part2>(A, max_n, fmt, warm, s);
     }
 }
 

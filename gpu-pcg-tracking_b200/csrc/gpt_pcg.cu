@@ -1810,7 +1810,7 @@ static cudaError_t launch_pcg_chain_cs(const BatchView &bv, int kpc_max, const v
 cudaError_t launch_pcg(const BatchView &bv, int max_n_knots, int min_n_knots, int fmt, int precond, const float *S,
                        const float *Pinv, const float *gamma, const double *gamma64, float *lambda,
                        double *lambda64, double *cr_ws, int max_iter, float tol, int exit_mode, uint32_t *out_iters,
-                       uint32_t *pcg_log, int log_stride, int cluster_size, int num_sms, cudaStream_t s)
+                       uint32_t *pcg_log, int log_stride, int cluster_size, int num_sms, cudaStream_t s, bool zero_start)
 {
     if (bv.B <= 0) return cudaSuccess;
     if (precond == 1 && !cr_ws) return cudaErrorInvalidValue;
@@ -1819,11 +1819,13 @@ cudaError_t launch_pcg(const BatchView &bv, int max_n_knots, int min_n_knots, in
     // The library's choice for packed rows and the exact preconditioner is the partitioned kernel: at every size
     // measured it is the fastest of the exact ones (us per launch, partitioned / one cyclic-reduction CTA: 1 x 32
     // 27 / 68, 11 x 77 42 / 144, 512 x 128 187 / 781; horizons past 128 knots, which cyclic reduction spreads
-    // over CTAs that iterate: 1 x 511 85 / 6167).  Rows in the reference's layout keep cyclic reduction below.
-    if (cluster_size == PCG_WARP_QUAD || (cluster_size == 0 && precond == 1 && fmt != 0)) {
+    // over CTAs that iterate: 1 x 511 85 / 6167).  Like every kernel but PCG_WARP_QUAD's by name it starts from the
+    // caller's lambda: one that meets the tolerance is kept.  Rows in the reference's layout keep cyclic reduction below.
+    const bool chosen = cluster_size == 0 && precond == 1 && fmt != 0;
+    if (cluster_size == PCG_WARP_QUAD || chosen) {
         if (precond != 1 || fmt == 0) return cudaErrorInvalidValue;  // packed rows, exact preconditioner
         return launch_pcg_part(bv, max_n_knots, fmt, S, gamma, gamma64, lambda, lambda64, cr_ws, max_iter, tol,
-                               exit_mode, out_iters, pcg_log, log_stride, num_sms, s);
+                               exit_mode, out_iters, pcg_log, log_stride, num_sms, s, chosen && !zero_start);
     }
     if (cluster_size == PCG_WARP_PAIR) {
         if (precond != 1 || fmt == 0) return cudaErrorInvalidValue;  // packed rows, exact preconditioner

@@ -124,8 +124,9 @@ typedef struct gpt_sqp_stats {
  * (partitioned block LDL^T: separator knots between the parts, whose reduced system two warps factor from both
  * ends), 2 to 32 of them on one CTA or a cluster of 2, 4 or 8, by the batch size and the longest horizon of the
  * call (few instances: more parts, a shorter chain; many: less work); same iteration and preconditioner (exact inverse of S) as
- * pcg_cluster_size 1.  The same batch gives the same bits; an instance's last bits may differ between
- * batches that run with another number of parts. */
+ * pcg_cluster_size 1.  Given by name it starts from lambda = 0, whatever d_lambda holds; as the library's choice (0) from
+ * d_lambda, which it returns unchanged, after no iteration, where it meets the tolerance.  The same batch gives the same
+ * bits; an instance's last bits may differ between batches that run with another number of parts. */
 #define GPT_PCG_WARP_QUAD 64u
 
 /* Default configs: the reference's logged experiment settings (dt 1/64, Euler,
