@@ -1554,20 +1554,27 @@ static gpt_status track_impl(gpt_handle *h, uint32_t B, const uint32_t *h_N, con
     }
     // An update's plant simulation needs the state and the previous update's controls only, so it runs on a stream of
     // its own beside the solve (it is a chain of plant steps, 80 us for 50 of them, on one warp per four
-    // instances); the update's shift waits for both.
+    // instances); the update's shift waits for both.  Two plant steps and fewer follow the solve: they take less than the
+    // events do (us an update beside / after it, 1 x 32 with two SQP iterations: no full step 159 / 157, two 161.4 / 160.8, four
+    // 159 / 166, 50 167 / 236; 512 x 64: 543 / 538, 544 / 542, 547 / 545, 602 / 623).
+    constexpr uint32_t SIM_BESIDE = 3;
+    const bool beside = tp.n_sub >= SIM_BESIDE;
     SimFork fork(h, s);
     for (uint32_t u = 0; u < n_updates; ++u) {
         GPT_CUDA(launch_track_prep(bv, h->trk_rows, h->trk_clk, tc.rho_reset, 0, s));
         GPT_CUDA(launch_track_clock(h->trk_clk, tp, s));
-        GPT_CUDA(fork.begin());
-        GPT_CUDA(launch_track_sim(bv, h->trk_rows, h->trk_clk, tp, d_xs, h->trk_xu_old, h->sim_stream));
+        if (beside) {
+            GPT_CUDA(fork.begin());
+            GPT_CUDA(launch_track_sim(bv, h->trk_rows, h->trk_clk, tp, d_xs, h->trk_xu_old, h->sim_stream));
+        }
         const gpt_status st = solve_on_workspace(h, plan, s);
         if (st != GPT_OK) return st;
         if (d_wgrad) {
             const gpt_status sa = enqueue_track_adjoint(h, plan, d_wgrad, d_loss, s);
             if (sa != GPT_OK) return sa;
         }
-        GPT_CUDA(fork.end());
+        if (beside) GPT_CUDA(fork.end());
+        else GPT_CUDA(launch_track_sim(bv, h->trk_rows, h->trk_clk, tp, d_xs, h->trk_xu_old, s));
         GPT_CUDA(launch_track_post(bv, h->trk_rows, h->trk_clk, d_eePos_traj, d_xu_traj, d_xs, h->gxu, h->trk_xu_old,
                                    h->ggoal, h->glam, h->adj_h, d_err, h->trk_inst, d_log, log_cap, s));
     }
