@@ -1137,7 +1137,7 @@ gpt_status gpt_autotune(gpt_handle *h, uint32_t B, const uint32_t *h_N, const fl
     std::vector<uint32_t> cand;
     for (int cs = cs0; cs <= 16 && cs <= 4 * cs0 && cs <= minN; cs *= 2) cand.push_back((uint32_t)cs);
     if (cand.empty()) cand.push_back((uint32_t)cs0);
-    if (h->sc.pcg_precond == 1) {  // one 128-thread CTA per instance: two or four factoring warps
+    if (h->sc.pcg_precond == 1) {  // the factorisations from both ends and in parts
         cand.push_back(GPT_PCG_WARP_PAIR);
         cand.push_back(GPT_PCG_WARP_QUAD);
     }
@@ -1201,7 +1201,9 @@ gpt_status gpt_autotune(gpt_handle *h, uint32_t B, const uint32_t *h_N, const fl
     // resident wave to the default 16 (a smaller grid gives each Schur warp a longer run of knots whose
     // inverses it reuses, and leaves no partial last wave); a change must gain 1 %
     static const uint8_t cta_cand[] = {4, 5, 6, 8};
+    const bool f64 = h->sc.pcg_precond == 1 && h->sc.schur_fp64;
     for (int which = 0; which < 4 && st == GPT_OK; ++which) {
+        if (which == 0 && f64 && kkt_lane(total, maxN)) continue;  // one knot per lane: no grid to choose
         uint8_t keep = cta[which];
         for (uint8_t cv : cta_cand) {
             cta[which] = cv;

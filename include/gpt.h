@@ -205,7 +205,7 @@ gpt_status gpt_sqp_solve_batched_trace(gpt_handle *h, uint32_t batch, const uint
  *      with pcg_precond 1, GPT_PCG_WARP_PAIR and GPT_PCG_WARP_QUAD;
  *   2. then, one kernel at a time, the grid of the per-knot kernels -- KKT formation, FP64 Schur complement,
  *      line-search merit, dz recovery -- as CTAs per SM in {4, 5, 6, 8, 16} (16 is the default; a change
- *      must gain 1 %);
+ *      must gain 1 %; the KKT kernel that takes one knot per lane has no such grid, and keeps 16);
  *   3. then, when the handle's sqp_graph is 1 (a graph solve whose branch count is left to the library),
  *      the part-batch branches per graph iteration in {1, 2, 4} (at most the batch; a change must gain
  *      1 %), which later graph solves of the shape use while sqp_graph stays 1.
