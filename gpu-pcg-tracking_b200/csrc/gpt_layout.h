@@ -11,7 +11,8 @@
 
 namespace gpt {
 
-constexpr int QUAD_NWARP = 4;
+// the variant of one CTA and four parts (Part4)
+constexpr int QUAD_NWARP = 4, QUAD_EDGE = 15;
 
 // NW: the most parts; edge: an edge part's length in tenths of a middle part's
 template <int NW>
@@ -66,6 +67,6 @@ GPT_HD inline PartLayout<NW> part_layout(int n, int edge)
 }
 
 using QuadLayout = PartLayout<QUAD_NWARP>;
-GPT_HD inline QuadLayout quad_layout(int n) { return part_layout<QUAD_NWARP>(n, 13); }
+GPT_HD inline QuadLayout quad_layout(int n) { return part_layout<QUAD_NWARP>(n, QUAD_EDGE); }
 
 }  // namespace gpt

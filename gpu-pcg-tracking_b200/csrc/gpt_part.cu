@@ -1112,7 +1112,7 @@ using Part32 = PartCfg<8, 4, 6, 1, 15>;
 using Part16 = PartCfg<4, 4, 6, 1, 15>;
 using Part8x2 = PartCfg<2, 4, 6, 1, 15>;
 using Part8 = PartCfg<1, 8, 6, 1, 15>;
-using Part4 = PartCfg<1, 4, 4, 2, 15>;
+using Part4 = PartCfg<1, QUAD_NWARP, 4, 2, QUAD_EDGE>;
 using Part2 = PartCfg<1, 2, 3, 4, 13>;
 
 // The variant of a batch.  More parts shorten an instance's chain but add the middle parts' work (about 1.6 of an edge

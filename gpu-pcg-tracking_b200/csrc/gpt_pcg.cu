@@ -1820,8 +1820,8 @@ cudaError_t launch_pcg(const BatchView &bv, int max_n_knots, int min_n_knots, in
     // measured it is the fastest of the exact ones (us per launch, partitioned / one cyclic-reduction CTA: 1 x 32
     // 27 / 68, 11 x 77 42 / 144, 512 x 128 187 / 781; horizons past 128 knots, which cyclic reduction spreads
     // over CTAs that iterate: 1 x 511 85 / 6167).  Like every kernel but PCG_WARP_QUAD's by name it starts from the
-    // caller's lambda: one that meets the tolerance is kept.  Rows in the reference's layout keep cyclic reduction below.
-    const bool chosen = cluster_size == 0 && precond == 1 && fmt != 0;
+    // caller's lambda: one that meets the tolerance is kept.
+    const bool chosen = cluster_size == 0 && precond == 1;
     if (cluster_size == PCG_WARP_QUAD || chosen) {
         if (precond != 1 || fmt == 0) return cudaErrorInvalidValue;  // packed rows, exact preconditioner
         return launch_pcg_part(bv, max_n_knots, fmt, S, gamma, gamma64, lambda, lambda64, cr_ws, max_iter, tol,
@@ -1836,7 +1836,7 @@ cudaError_t launch_pcg(const BatchView &bv, int max_n_knots, int min_n_knots, in
     }
     if (precond == 2 && fmt != 0) return cudaErrorInvalidValue;  // the stair Pinv comes in the reference layout
     const int kpc_cap = precond == 2 ? PCG_KPC_STAIR : PCG_KPC_MAX;
-    int cs = (precond == 1 && cluster_size == 0) ? 1 : pcg_pick_cluster(max_n_knots, bv.B, num_sms, cluster_size);
+    int cs = pcg_pick_cluster(max_n_knots, bv.B, num_sms, cluster_size);
     while ((max_n_knots + cs - 1) / cs > kpc_cap) cs *= 2;
     while (cs > 1 && cs > min_n_knots) cs /= 2;  // every CTA owns at least one knot
     const int kpc_max = (max_n_knots + cs - 1) / cs;
