@@ -94,6 +94,17 @@ __device__ __forceinline__ int tri_idx(int r, int c)  // packed lower triangle, 
 }
 __device__ __forceinline__ int inv_idx(int i, int c) { return 2 * (i >> 1) * ((i >> 1) + 1) + 2 * c + (i & 1); }
 
+// Reciprocal by one third-order step r (1 + e + e^2), e = 1 - x r, from the PTX approximation
+// rcp.approx.ftz.f64: a seed of relative error 2^-20 gives 2^-60 before rounding, in three dependent
+// operations (two Newton steps need four)
+__device__ __forceinline__ double rcp_cubic(double x)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
 // rows 2t, 2t + 1 (v0, v1) of a column, from this lane's own row and its partner's
 __device__ __forceinline__ void pair_rows(double own, double other, int h, double &v0, double &v1)
 {
@@ -104,9 +115,7 @@ __device__ __forceinline__ void pair_rows(double own, double other, int h, doubl
 // One elimination step on the lane layout above.  In: a = D (columns 14, 15: anything finite), e = [E^T | y | 0],
 // b = [A' | y' | 0].  Out: a = L^{-1} with the 2 x 2 blocks of B^{-1} on its diagonal (lower part), e = [W | z],
 // b -= W^T B^{-1} [W | z].  buf: QROWS_D doubles.  Seven block pivots of about 120 cycles each when the warp
-// is alone on its scheduler (the chain of two shared-memory trips and a reciprocal, correctly rounded but for some 1e-8 of
-// its arguments: a third-order step from the same seed, 3 in 10,000 off by a unit in the last place, saves 0.3 % of a
-// solve at 512 x 128).
+// is alone on its scheduler (the chain of two shared-memory trips and a reciprocal).
 __device__ __forceinline__ void part_step(double (&a)[7], double (&e)[7], double (&b)[7], double *buf, int lane)
 {
     const int c = lane >> 1, h = lane & 1;
@@ -121,7 +130,7 @@ __device__ __forceinline__ void part_step(double (&a)[7], double (&e)[7], double
         __syncwarp();
         const double x = bk[t].x, y = bk[9 + t].x, z = bk[27 + t].x;  // the pivot block
         const double2 op = bk[18 * (h ^ 1) + pos];
-        const double rd = rcp_newton(fma(x, z, -y * y));
+        const double rd = rcp_cubic(fma(x, z, -y * y));
         const double i00 = z * rd, i01 = -y * rd, i11 = x * rd;
         const bool p0 = c == 2 * t, p1 = c == 2 * t + 1, piv = p0 || p1;
         // this column's pivot rows (the identity's in the pivot columns) times B^{-1}
@@ -169,7 +178,7 @@ __device__ __forceinline__ void part_step_mid(double (&a)[7], double (&e)[7], do
         const double x = bk[t], y = bk[8 + t], z = bk[24 + t];
         const double ap = bk[16 * (h ^ 1) + pos], ep = W[(2 * t + (h ^ 1)) * QLD + c],
                      fp = vbuf[(2 * t + (h ^ 1)) * QLD + c];
-        const double rd = rcp_newton(fma(x, z, -y * y));
+        const double rd = rcp_cubic(fma(x, z, -y * y));
         const double i00 = z * rd, i01 = -y * rd, i11 = x * rd;
         if (c == 0) *reinterpret_cast<double2 *>(binv + 2 * (2 * t + h)) = make_double2(h ? i11 : i00, i01);
         const bool p0 = c == 2 * t, p1 = c == 2 * t + 1, piv = p0 || p1;
