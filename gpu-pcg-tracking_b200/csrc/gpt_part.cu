@@ -94,17 +94,6 @@ __device__ __forceinline__ int tri_idx(int r, int c)  // packed lower triangle, 
 }
 __device__ __forceinline__ int inv_idx(int i, int c) { return 2 * (i >> 1) * ((i >> 1) + 1) + 2 * c + (i & 1); }
 
-// Reciprocal by one third-order step r (1 + e + e^2), e = 1 - x r, from the PTX approximation
-// rcp.approx.ftz.f64: a seed of relative error 2^-20 gives 2^-60 before rounding, in three dependent
-// operations (two Newton steps need four)
-__device__ __forceinline__ double rcp_cubic(double x)
-{
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    const double e = fma(-x, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-
 // rows 2t, 2t + 1 (v0, v1) of a column, from this lane's own row and its partner's
 __device__ __forceinline__ void pair_rows(double own, double other, int h, double &v0, double &v1)
 {

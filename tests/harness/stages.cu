@@ -75,3 +75,19 @@ extern "C" int stage_kkt(int batch, const int *h_off, const unsigned char *h_act
     const ProblemParams P{dt, integrator, 1.f, qd_cost, r_cost, 10.f, ref_terminal};
     return v.done(launch_kkt(v.bv, P, xu, goal, xs, nullptr, C, g, c, sms(), 0, 16, KKT_G_NONE));
 }
+
+namespace {
+__global__ void rcp_kernel(int n, int order, const double *x, double *r)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        r[i] = order == 3 ? rcp_cubic(x[i]) : rcp_newton(x[i]);
+}
+}  // namespace
+
+// the kernels' FP64 reciprocals of each x: order 2 by two Newton-Raphson steps, 3 by one third-order step
+extern "C" int stage_rcp(int n, int order, const double *x, double *r)
+{
+    rcp_kernel<<<256, 256>>>(n, order, x, r);
+    const cudaError_t e = cudaGetLastError();
+    return (int)(e != cudaSuccess ? e : cudaDeviceSynchronize());
+}
