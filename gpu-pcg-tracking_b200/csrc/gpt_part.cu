@@ -66,7 +66,7 @@ constexpr int QLD = 20;                    // leading dimension of W and V (conf
 constexpr int QW_D = NS * QLD;             // W or V (14 rows x 16 columns)
 constexpr int QROWS_D = 2 * 2 * 37;        // pivot rows: 2 sets of 2 rows (D, E^T), 37 pairs apart
 constexpr int QBUF = QROWS_D + 2 * NS;     // pivot rows; B^{-1} by rows
-constexpr int RED_N = 4;                   // values of a reduction
+constexpr int RED_N = 3;                   // values of a reduction, and one more apart from them (the start's check)
 constexpr int RR_PERIOD = 32;              // CG iterations between true-residual replacements
 
 // A kernel variant: a cluster of CL CTAs of WC warps per instance (NW = CL WC parts, in order over the CTAs), SL staging
@@ -84,7 +84,7 @@ struct PartCfg {
     static constexpr int MID = MIDS * QW_D > SEP_SX + WC * NS ? MIDS * QW_D : SEP_SX + WC * NS;
     static size_t smem_bytes(int n)
     {
-        return sizeof(double) * (size_t)(NS * n + WC * (REGION + QBUF) + MID + 2 * NW * RED_N + 4);
+        return sizeof(double) * (size_t)(NS * n + WC * (REGION + QBUF) + MID + 2 * NW * (RED_N + 1) + 4);
     }
 };
 
@@ -330,9 +330,9 @@ struct PartSmem {
         stg = base;                         // per warp: staged rows / steps; the separators' blocks
         buf = stg + CF::WC * CF::REGION;    // per warp: pivot rows; the backward sweep's scratch
         wmid = buf + CF::WC * QBUF;
-        red = wmid + CF::MID;               // 2 sets x NW warps x RED_N
-        lay = reinterpret_cast<int *>(red + 2 * CF::NW * RED_N);  // parts, first separator, spacing, this CTA's knots
-        xv = red + 2 * CF::NW * RED_N + 4;  // 14 n: y, then z, then x (of the CTA's knots and all separators)
+        red = wmid + CF::MID;               // 2 sets x NW warps x RED_N, 2 sets x NW warps
+        lay = reinterpret_cast<int *>(red + 2 * CF::NW * (RED_N + 1));  // parts, first separator, spacing, this CTA's knots
+        xv = red + 2 * CF::NW * (RED_N + 1) + 4;  // 14 n: y, then z, then x (of the CTA's knots and all separators)
     }
 };
 
@@ -485,7 +485,7 @@ struct PartArgs {
     const double *gamma64;
     float *lambda;
     double *lambda64, *ws;
-    int max_iter, exit_mode, log_stride;
+    int max_iter, exit_mode, log_stride, warm;
     float tol;
     uint32_t *out_iters, *pcg_log;
 };
@@ -554,10 +554,10 @@ __device__ __noinline__ double part_start_bound(const PartArgs &A, int w, int nw
     return h == 0 && c < NS ? fma(r, r, s) : s;
 }
 
-// y in xv -> x of M x = y in xv, and S x in the workspace (QW_SX); WARM and check: bound as of part_start_bound, by the
+// y in xv -> x of M x = y in xv, and S x in the workspace (QW_SX); CHECK and first: bound as of part_start_bound, by the
 // warps that wait for the separators
-template <int FMT, class CF, bool WARM>
-__device__ __forceinline__ void part_apply(const PartArgs &A, bool check, double &bound)
+template <int FMT, class CF, bool CHECK>
+__device__ __forceinline__ void part_apply(const PartArgs &A, bool first, double &bound)
 {
     using ST = typename PartRows<FMT>::ST;
     constexpr int NW = CF::NW;
@@ -680,7 +680,7 @@ __device__ __forceinline__ void part_apply(const PartArgs &A, bool check, double
             }
         }
     }
-    if (WARM && check) {
+    if (CHECK && first) {
         const int w0 = rank == 0 && P >= 2 ? (NW == 2 ? 1 : 2) : 0;
         if (warp >= w0) bound = part_start_bound<FMT, CF>(A, warp - w0, CF::WC - w0);
     }
@@ -805,20 +805,21 @@ __device__ __forceinline__ void part_apply(const PartArgs &A, bool check, double
 template <class CF, int CNT, int LEN>
 __device__ __forceinline__ void part_sum(double (&v)[LEN], int set)
 {
-    static_assert(CNT <= LEN && CNT <= RED_N, "the reduction's slots");
+    static_assert(CNT <= LEN && CNT <= RED_N + 1, "the reduction's slots");
     extern __shared__ __align__(16) double part_dyn_smem[];
-    double *red = PartSmem<CF>(part_dyn_smem).red + set * CF::NW * RED_N;
+    double *all = PartSmem<CF>(part_dyn_smem).red, *red = all + set * CF::NW * RED_N;
+    double *more = all + (2 * RED_N + set) * CF::NW;
     const int lane = threadIdx.x & 31, part = part_rank<CF>() * CF::WC + (threadIdx.x >> 5);
 #pragma unroll
     for (int q = 0; q < CNT; ++q) {
         const double s = warp_sum(v[q]);
-        if (lane < CF::CL) part_peer<CF>(red, lane)[RED_N * part + q] = s;
+        if (lane < CF::CL) *part_peer<CF>(q < RED_N ? red + RED_N * part + q : more + part, lane) = s;
     }
     part_sync<CF>();
 #pragma unroll
     for (int q = 0; q < CNT; ++q) {
         double s = 0.0;
-        for (int w = 0; w < CF::NW; ++w) s += red[RED_N * w + q];
+        for (int w = 0; w < CF::NW; ++w) s += q < RED_N ? red[RED_N * w + q] : more[w];
         v[q] = s;
     }
 }
@@ -868,9 +869,12 @@ __device__ __noinline__ double part_true_residual(const PartArgs &A, int set, bo
     return s[0];
 }
 
-// WARM: from the caller's lambda (a kernel of its own: the code for it costs the one that starts from 0 nine us of 187 at
-// 512 x 128)
-template <int FMT, class CF, bool WARM>
+// CHECK: a caller's lambda that meets the tolerance is the result.  Any other leads to the solution from 0 too, so whether it
+// does is told by a part of its residual, formed by warps that wait for the separators, and by all of it only where that
+// part does not exclude it: a residual ahead of the elimination took 3.6 us more a launch at 32 knots (27 us in all) and 62
+// at 512 x 128 (186), the part takes 0 and 12.  (A kernel of its own: its code costs the one that starts from 0 nine us at
+// 512 x 128.)  A.warm without CHECK iterates from the caller's lambda.
+template <int FMT, class CF, bool CHECK>
 __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const __grid_constant__ PartArgs A)
 {
     static_assert(FMT == 1 || FMT == 2, "packed rows only");
@@ -878,11 +882,6 @@ __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const _
     extern __shared__ __align__(16) double part_dyn_smem[];
     double *xv = PartSmem<CF>(part_dyn_smem).xv;
     const int tid = threadIdx.x;
-    // A given start that does not meet the tolerance leads to the solution from 0 too.  Whether it does is told by a part of
-    // its residual, formed by warps that wait for the separators, and by all of it only where that part does not exclude
-    // it: a residual ahead of the elimination took 3.6 us more a launch at 32 knots (27 us in all) and 62 at 512 x 128
-    // (187), the part takes 0 and 12.  The exit test on r . z, or no iteration at all, takes the start as it is.
-    const bool check = WARM && A.exit_mode == 0 && A.max_iter > 0;
     {
         const PartCtx<FMT, CF> cx(A);
         if (!A.bv.active(cx.inst)) return;  // (the whole cluster)
@@ -908,7 +907,7 @@ __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const _
     bool conv = false, bad = false, in_xv = false;
     bool has_res = false;  // r and lambda are in the workspace (before: r = gamma, lambda = 0)
     double eta = 0.0, gg = 0.0, alpha = 0.0;
-    if (WARM && !check) {
+    if (A.warm) {
         part_sync<CF>();
         const PartCtx<FMT, CF> cx(A);
         const PartRange<CF> rg;
@@ -934,7 +933,7 @@ __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const _
     };
     for (;;) {
         double bound = 0.0;
-        part_apply<FMT, CF, WARM>(A, check && it == 0, bound);
+        part_apply<FMT, CF, CHECK>(A, it == 0, bound);
         const PartCtx<FMT, CF> cx(A);
         const PartRange<CF> rg;
         double dd[4] = {0.0, 0.0, 0.0, bound};  // r . z, r . r with z = -x; x . S x; the start's bound
@@ -960,12 +959,12 @@ __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const _
             if (rg.first + NT * i < rg.end) dots(rk[i], xv[rg.first + NT * i], sk[i]);
         for (int e = rg.first + NT * KEEP; e < rg.end; e += NT)
             dots(has_res ? cx.vec(QW_RES, e) : cx.gam(e), xv[e], cx.vec(QW_SX, e));
-        part_sum<CF, WARM ? 4 : 3>(dd, set);
+        part_sum<CF, CHECK ? 4 : 3>(dd, set);
         set ^= 1;
         if (it == 0) {
             if (!has_res) gg = dd[1];
-            conv = check ? gg == 0.0 : converged(dd[0], dd[1]);
-            if (check && !conv && !(dd[3] > (double)A.tol * (double)A.tol * gg)) {
+            conv = CHECK ? gg == 0.0 : converged(dd[0], dd[1]);
+            if (CHECK && !conv && !(dd[3] > (double)A.tol * (double)A.tol * gg)) {
                 const double r0 = part_true_residual<FMT, CF>(A, set, true);
                 set ^= 1;
                 bad = !isfinite(r0);
@@ -1082,10 +1081,10 @@ __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const _
     }
 }
 
-template <int FMT, class CF, bool WARM>
+template <int FMT, class CF, bool CHECK>
 static cudaError_t launch_part_t(const PartArgs &A, int max_n, cudaStream_t s)
 {
-    auto kern = pcg_part_kernel<FMT, CF, WARM>;
+    auto kern = pcg_part_kernel<FMT, CF, CHECK>;
     const size_t smem = CF::smem_bytes(max_n);
     const cudaError_t e = ensure_func_attrs((const void *)kern, smem);
     if (e != cudaSuccess) return e;
@@ -1134,9 +1133,9 @@ int part_variant(int B, int max_n, int num_sms)
 }
 
 template <class CF>
-static cudaError_t launch_part_f(const PartArgs &A, int max_n, int fmt, bool warm, cudaStream_t s)
+static cudaError_t launch_part_f(const PartArgs &A, int max_n, int fmt, bool check, cudaStream_t s)
 {
-    if (warm) return fmt == 2 ? launch_part_t<2, CF, true>(A, max_n, s) : launch_part_t<1, CF, true>(A, max_n, s);
+    if (check) return fmt == 2 ? launch_part_t<2, CF, true>(A, max_n, s) : launch_part_t<1, CF, true>(A, max_n, s);
     return fmt == 2 ? launch_part_t<2, CF, false>(A, max_n, s) : launch_part_t<1, CF, false>(A, max_n, s);
 }
 
@@ -1145,15 +1144,17 @@ cudaError_t launch_pcg_part(const BatchView &bv, int max_n, int fmt, const void 
                             float tol, int exit_mode, uint32_t *out_iters, uint32_t *pcg_log, int log_stride,
                             int num_sms, cudaStream_t s, bool warm)
 {
+    // the exit test on r . z, and no iteration at all, take the start as it is
+    const bool check = warm && exit_mode == 0 && max_iter > 0;
     const PartArgs A{bv,       S,         gamma,      gamma64, lambda,    lambda64, ws,
-                     max_iter, exit_mode, log_stride, tol, out_iters, pcg_log};
+                     max_iter, exit_mode, log_stride, warm && !check ? 1 : 0, tol, out_iters, pcg_log};
     switch (bv.part_variant ? bv.part_variant : part_variant(bv.B, max_n, num_sms)) {
-    case PART_32: return launch_part_f<Part32>(A, max_n, fmt, warm, s);
-    case PART_16: return launch_part_f<Part16>(A, max_n, fmt, warm, s);
-    case PART_8X2: return launch_part_f<Part8x2>(A, max_n, fmt, warm, s);
-    case PART_8: return launch_part_f<Part8>(A, max_n, fmt, warm, s);
-    case PART_4: return launch_part_f<Part4>(A, max_n, fmt, warm, s);
-    default: return launch_part_f<Part2>(A, max_n, fmt, warm, s);
+    case PART_32: return launch_part_f<Part32>(A, max_n, fmt, check, s);
+    case PART_16: return launch_part_f<Part16>(A, max_n, fmt, check, s);
+    case PART_8X2: return launch_part_f<Part8x2>(A, max_n, fmt, check, s);
+    case PART_8: return launch_part_f<Part8>(A, max_n, fmt, check, s);
+    case PART_4: return launch_part_f<Part4>(A, max_n, fmt, check, s);
+    default: return launch_part_f<Part2>(A, max_n, fmt, check, s);
     }
 }
 
