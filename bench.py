@@ -43,7 +43,7 @@ PCG_BJ_BYTES_PER_KNOT = 4 * 784  # block-Jacobi kernel: FP32 S (588) + Pinv (196
 # the bench's batch, 512 instances x 128 knots (the working set of a launch, ~0.26 GB, exceeds the L2, so
 # the traffic per knot depends on the batch and is not scaled to other batches)
 PCG_DRAM_BYTES_PER_KNOT = {"pcg_pair_kernel": (779.677440e6 + 92.534528e6) / (512 * 128),
-                           "pcg_part_kernel": (355.878912e6 + 70.890240e6) / (512 * 128)}
+                           "pcg_part_kernel": (356.141824e6 + 68.516096e6) / (512 * 128)}
 PCG_DRAM_SOURCE = "ncu capture of the 512 x 128 bench batch, one launch"
 ALG_FLOATS_PER_KNOT_SQP = 4058   # every materialised SQP-iteration tensor written once, read once
 
@@ -476,7 +476,8 @@ def fp64_accuracy(gpt, sv, Ns, batch, n_inst, iters):
     the KKT blocks at each recorded iterate come from gpt_form_kkt, the FP64 Schur complement, block
     Cholesky and dz from fp64check): of the whole batch, whose KKT blocks (a knot per lane) differ from
     gpt_form_kkt's by FP32 rounding, and of the sampled instances as a batch of their own, which forms
-    the same blocks, so that the difference is the solver's alone."""
+    the same blocks, so that the difference is the solver's alone -- with the PCG variant of that small
+    batch, not the timed one's (the tests hold each variant, and the lane form's blocks, against FP64)."""
     import numpy as np
     import torch
     F = importlib.import_module("gpu-pcg-tracking_b200.fp64check")
@@ -510,7 +511,9 @@ def fp64_accuracy(gpt, sv, Ns, batch, n_inst, iters):
             for k, w in (("xu", 21), ("goal", 6), ("lam", 14))}
     s_lam, s_dz, _ = errors([Ns[b] for b in sample], part, range(len(sample)))
     return {"lambda_max_rel_err": e_lam, "dz_max_rel_err": e_dz, "iterates": n, "instances": sample,
-            "sample_alone": {"lambda_max_rel_err": s_lam, "dz_max_rel_err": s_dz},
+            "sample_alone": {"lambda_max_rel_err": s_lam, "dz_max_rel_err": s_dz,
+                             "kernels": f"those of a batch of {len(sample)}: KKT by half-warps, the partitioned PCG "
+                                        "with more parts per instance than in the timed batch"},
             "reference": "FP64 host Schur complement + block Cholesky + dz of gpt_form_kkt's blocks at each recorded "
                          "iterate (max |err| / max |FP64|); the whole batch's own blocks differ from these by FP32 "
                          "rounding, those of the sampled instances alone do not"}

@@ -441,8 +441,10 @@ __global__ void __launch_bounds__(32 * KKTL_WARPS, 8 / KKTL_WARPS)
 
 // One knot per lane from 9216 knots on: up to four warps per SM (18,944 knots) a launch of that form takes 29 to 36 us, the
 // half-warp form 25.8 at 6,192 knots, 30 at 8,256, 39.4 at 12,384 and 49.2 at 16,512; at 65,536 the two take 70 and
-// 170 us.  The two differ by FP32 rounding, which a solve amplifies with its horizon (a step's multipliers at 128 knots by
-// 1e-6 of their size, at 511 knots by 3e-5), so longer horizons stay with the half-warp form, whose results they have.
+// 170 us.  The two differ by FP32 rounding (each as far from the FP64 blocks, 1.4e-7 and 1.5e-7 root mean square of the
+// largest entry of d/dq; a step's multipliers differ by up to 2e-6 of their largest, median 1e-7 to 5e-7, at horizons of 32
+// to 511 alike).  The line at 128 knots is not one of speed or rounding: it is how far the lane form's solves are held against
+// FP64, so longer horizons keep the half-warp form and its bits.
 bool kkt_lane(int total_knots, int max_n) { return total_knots >= 9216 && max_n <= 128; }
 
 cudaError_t launch_kkt(const BatchView &bv, const ProblemParams &P, const float *xu, const float *goal,

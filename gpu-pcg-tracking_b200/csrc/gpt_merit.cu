@@ -25,7 +25,7 @@ constexpr int DZ_WARPS = 4;
 // block, the velocity and control diagonals -- a quarter of the full layout's bytes).  The sums are those of
 // the full layout term by term (the skipped terms are exact zeros).  512 x 128 knots: 43 us with a branch for
 // the states and one for the controls, 36 this way (129 MB, 20 us; now
-// the L1 pipe is 72 % busy); loading a knot ahead of the previous one's
+// the L1 pipe is 78 % busy); loading a knot ahead of the previous one's
 // arithmetic gave nothing.
 template <bool COMPACT>
 struct __align__(16) DzWarpSmem {

@@ -24,8 +24,8 @@
 //   x_k = L^{-T} B^{-1} (z_k + L^{-1} t),  t = -E^T x_next - F_k x_left.
 // The pivots run on the FP64 pipe with the pivot rows broadcast through shared memory; the rank-14
 // products of a middle part on the FP64 tensor cores (part_step_mid).  What bounds a step is the length of its
-// dependent chain and the instructions around it: issue is 0.3 to 0.45 per cycle and scheduler, the FP64
-// pipe 20 % busy, shared memory 39 % (ncu).
+// dependent chain and the instructions around it: at 512 x 128 issue is 0.41 per cycle and scheduler, the FP64
+// pipe 23 % and the L1 and shared-memory pipe 66 % busy (ncu).
 //
 // A preconditioner application is one such factorisation: with an exact preconditioner the iteration
 // almost always ends after the first, so nothing but L^{-1} and F is kept for another right-hand side.

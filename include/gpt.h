@@ -165,7 +165,11 @@ gpt_status gpt_sqp_solve(gpt_handle *h, uint32_t knot_points, const float *d_eeP
 
 /* Many independent instances of uneven horizon in one call (no reference
  * counterpart; the reference solves one instance per sqpSolve).  h_rho and
- * h_stats have `batch` entries. */
+ * h_stats have `batch` entries.
+ * An instance's result does not depend on the other instances' data, but its last bits may on the batch's shape, which
+ * chooses the kernels: the parts of the PCG (GPT_PCG_WARP_QUAD above) by the number of instances and the longest horizon,
+ * and the KKT formation, one knot per lane (sums in another order) for batches of 9216 knots and more whose longest
+ * horizon is at most 128 knots.  The same holds for the tracking calls and the adjoints. */
 gpt_status gpt_sqp_solve_batched(gpt_handle *h, uint32_t batch, const uint32_t *h_knot_points,
                                  const float *d_eePos_traj, float *d_lambda, float *d_xu, float *h_rho,
                                  float rho_reset, gpt_sqp_stats *h_stats, gpt_stream_t stream);
