@@ -1057,7 +1057,9 @@ __global__ void __launch_bounds__(32 * CF::WC, CF::MINB) pcg_part_kernel(const _
     const PartCtx<FMT, CF> cx(A);
     const PartRange<CF> rg;
     for (int e = rg.first; e < rg.end; e += NT) {
-        const double lam = in_xv ? -alpha * xv[e] : (has_res ? cx.vec(QW_LAM, e) : 0.0);
+        // CHECK: a system that is not finite leaves the start
+        const double none = CHECK && bad ? (double)A.lambda[NS * cx.kg0 + e] : 0.0;
+        const double lam = in_xv ? -alpha * xv[e] : (has_res ? cx.vec(QW_LAM, e) : none);
         A.lambda[NS * cx.kg0 + e] = (float)lam;
         if (A.lambda64) A.lambda64[NS * cx.kg0 + e] = lam;
     }

@@ -54,3 +54,23 @@ def test_the_given_lambda_is_where_the_solve_starts(problem_mod, Ns, schur_fp64,
     first[-1] = np.nan
     with pytest.raises(gpt.GptError):
         solve(first, 1e-6, 20)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("N", [5, 33, 129, 300])
+@pytest.mark.parametrize("at", [0.3, 0.5, 0.99])
+def test_a_system_that_is_not_finite_leaves_the_start(N, at):
+    """gpt_pcg reports a NaN in S, wherever it is, and returns the lambda that it was given."""
+    import torch
+    gpt = importlib.import_module("gpu-pcg-tracking_b200")
+    S = torch.zeros(N, 3, 14, 14, device="cuda")
+    S[:, 1] = -2.0 * torch.eye(14, device="cuda")
+    S[int(at * N), 1] = float("nan")
+    gam, lam = torch.ones(14 * N, device="cuda"), torch.arange(14.0 * N, device="cuda")
+    lam64 = torch.zeros(14 * N, device="cuda", dtype=torch.float64)
+    want = lam.clone()
+    sv = gpt.Solver(max_knot_points=N, timestep=0.01, integrator=1, qd_cost=1e-2, r_cost=1e-4)
+    with pytest.raises(gpt.GptError):
+        sv.pcg(N, S.reshape(-1), torch.zeros_like(S).reshape(-1), gam, lam, 20, 1e-6, 0, lam64=lam64)
+    assert torch.equal(lam, want) and torch.equal(lam64, want.double())
+    sv.close()
